@@ -1176,22 +1176,24 @@ static int ensure_fl_scratch(Ctx* c, size_t n) {
   return RAPT_OK;
 }
 
-// BounceCenter passes. A first pass gives each thread a small trace slot
+// BounceCenter passes. A first pass gives each line small trace slots
 // (kBcCapSmall points per direction: 8 KB; the lines of the pitch angles where
-// the reference's second-invariant integral runs have a few tens), 16,384
-// tracers at a time, so that the slots (128 MiB) stay in L2; a tracer whose
+// the reference's second-invariant integral runs have a few tens), 4,096
+// tracers at a time: 65,536 lanes, enough to fill the chip, and 200 MB of
+// slots of which the short lines touch an L2-sized part. A tracer whose
 // right-hand side met a non-finite value (a trace that did not fit, among
 // others) is then rerun from its start with full slots (kFieldlineCap points,
-// 64 KB), 2,048 at a time. The rerun reproduces a full-slot run exactly.
+// 64 KB), 512 at a time. The rerun reproduces a full-slot run exactly.
 constexpr int kBcCapSmall = 128;
-constexpr int64_t kBcChunkSmall = 16384, kBcChunkFull = 2048;
+constexpr int64_t kBcChunkSmall = 4096, kBcChunkFull = 512;
+constexpr int64_t kBcEvalChunk = 2048;  // rapt_bc_eval: one thread and one full slot a point
 
 static int bc_pass(Ctx* c, int64_t n, double* state, const double* cst, double delta, double bctimestep,
                    double eyegradientstep, double* rows, int32_t max_rows, int32_t* nrows, int32_t* status,
                    int64_t* counters, int32_t* flagged, int cap, int64_t chunk_max) {
   const long long stride = 8LL * cap;
   const int64_t chunk = std::min<int64_t>(n, chunk_max);
-  int rc = ensure_fl_scratch(c, (size_t)chunk * (size_t)cap / kFieldlineCap + 1);
+  int rc = ensure_fl_scratch(c, (size_t)bc_trace_slots(chunk) * (size_t)cap / kFieldlineCap + 1);
   if (rc) return rc;
   KParams P = make_params(c, RAPT_KIND_GC);
   const ModelTable& T = c->tab[c->field.model];
@@ -1298,7 +1300,7 @@ int rapt_bc_eval(void* ctx, int what, int64_t n, const double* tpos, const doubl
   if (n == 0) return RAPT_OK;
   CK(cudaSetDevice(c->device));
   const long long stride = 8LL * kFieldlineCap;
-  const int64_t chunk = std::min<int64_t>(n, kBcChunkFull);
+  const int64_t chunk = std::min<int64_t>(n, kBcEvalChunk);
   int rc = ensure_fl_scratch(c, (size_t)chunk);
   if (rc) return rc;
   const size_t C = (size_t)chunk;

@@ -8,11 +8,10 @@
 //   flutils.halfbouncepath          rapt/flutils.py:254-316
 //   Fieldline.trace with rkf        rapt/fieldline.py:13-107, rapt/rkf.py:13-143
 // and the SciPy routines halfbouncepath calls, from their published methods:
-// the quadratic interpolating B-spline of interp1d(kind='quadratic') and
-// Brent's root finder (brentq defaults); the final integral (quad in the
-// reference) is taken to convergence (see fl_bounce_integral). Products and
-// sums are rounded separately (no FMA contraction), as the reference's numpy
-// arithmetic is.
+// the quadratic interpolating B-spline of interp1d(kind='quadratic'), its
+// mirror points (the panels' roots; Brent's method where the line is not one
+// well) and the integral between them, taken exactly where the reference calls
+// quad (fl_well; fl_bounce_integral for the other lines).
 //
 // The (s, |B|) samples of the trace live in a per-thread scratch buffer:
 // the backward half written downwards from slot cap, the forward half upwards,
@@ -58,24 +57,31 @@ __device__ double fl_curvature(const FieldP& f, double t, const double* X) {
   return sqrt(ndot3(gp, gp)) / B;
 }
 
-// d[s,x,y,z]/ds = sign (1, b) (fieldline.py:39-51)
+// One direction of Fieldline.trace (fieldline.py:53-105): repeated rkf(f, 0, ds,
+// x0, tol, hmax = ds, hmin = 1e-6) calls (rkf.py:13-143) along sign b from X
+// until |B| > Bm. Accepted points go to slots idx, idx + dirn, ... (arc length
+// and |B|); where rkf raises, the reference keeps none of that call's points
+// (fieldline.py:68-69) and the trace ends. overflow: the buffer is full, or the
+// field is not finite (the caller's answer is NaN either way).
+//
+// Every stored value is the reference's bit for bit (products and sums rounded
+// separately, quotients by |B|): the second invariant's differences, and the
+// step sizes chosen on them, see the trace's last bits. What the reference's
+// arithmetic repeats is formed once: an accepted point's field is also the next
+// step's first stage; the arc length's slope is +-1 and its error estimate
+// zero; the step factor 0.84 (tol / r)^(1/4), which the cap hmax cuts off as
+// long as r is under about half of tol, is evaluated only where it can matter.
 template <int M>
-__device__ __forceinline__ void fl_deriv(const FieldP& f, double t, double sign, const double* Y, double* o) {
+__device__ __forceinline__ void fl_unit(const FieldP& f, double t, const double* X, double* u, double& mag) {
   double B[3];
-  Field<M>::B(f, t, Y[1], Y[2], Y[3], B);
-  const double m = sqrt(ndot3(B, B));
-  o[0] = sign;
-  o[1] = sign > 0 ? B[0] / m : -(B[0] / m);
-  o[2] = sign > 0 ? B[1] / m : -(B[1] / m);
-  o[3] = sign > 0 ? B[2] / m : -(B[2] / m);
+  Field<M>::B(f, t, X[0], X[1], X[2], B);
+  mag = sqrt(ndot3(B, B));
+  u[0] = B[0] / mag; u[1] = B[1] / mag; u[2] = B[2] / mag;
 }
 
-// rkf(f, 0, b, x0, tol, hmax, hmin) (rkf.py:13-143). Accepted points go to
-// slots idx, idx + dirn, ... (s and |B|); returns false where rkf raises (the
-// trace then ends) and sets overflow when the buffer is full.
 template <int M>
-__device__ bool fl_rkf(const FieldP& f, double t0, double sign, double* x, double b, double tol, double hmax,
-                       double hmin, double* S, double* Bs, int& idx, int dirn, int lo, int hi, bool& overflow) {
+__device__ __noinline__ int fl_trace_dir(const FieldP& f, double t0, const double* X, double Bm, double ds,
+                                         bool forward, double* S, double* Bs, int cap, bool& overflow) {
   constexpr double b21 = 2.500000000000000e-01, b31 = 9.375000000000000e-02, b32 = 2.812500000000000e-01,
                    b41 = 8.793809740555303e-01, b42 = -3.277196176604461e+00, b43 = 3.320892125625853e+00,
                    b51 = 2.032407407407407e+00, b52 = -8.000000000000000e+00, b53 = 7.173489278752436e+00,
@@ -85,49 +91,74 @@ __device__ bool fl_rkf(const FieldP& f, double t0, double sign, double* x, doubl
                    r5 = 2.000000000000000e-02, r6 = 3.636363636363636e-02;
   constexpr double c1 = 1.157407407407407e-01, c3 = 5.489278752436647e-01, c4 = 5.353313840155945e-01,
                    c5 = -2.000000000000000e-01;
-  double t = 0.0, h = hmax;
-  for (int guard = 0; guard < 100000 && t < b; ++guard) {
-    if (da(t, h) > b) h = da(b, -t);
-    double k1[4], k2[4], k3[4], k4[4], k5[4], k6[4], xt[4], fv[4];
-    fl_deriv<M>(f, t0, sign, x, fv);
-    for (int i = 0; i < 4; ++i) k1[i] = dm(h, fv[i]);
-    for (int i = 0; i < 4; ++i) xt[i] = da(x[i], dm(b21, k1[i]));
-    fl_deriv<M>(f, t0, sign, xt, fv);
-    for (int i = 0; i < 4; ++i) k2[i] = dm(h, fv[i]);
-    for (int i = 0; i < 4; ++i) xt[i] = da(da(x[i], dm(b31, k1[i])), dm(b32, k2[i]));
-    fl_deriv<M>(f, t0, sign, xt, fv);
-    for (int i = 0; i < 4; ++i) k3[i] = dm(h, fv[i]);
-    for (int i = 0; i < 4; ++i) xt[i] = da(da(da(x[i], dm(b41, k1[i])), dm(b42, k2[i])), dm(b43, k3[i]));
-    fl_deriv<M>(f, t0, sign, xt, fv);
-    for (int i = 0; i < 4; ++i) k4[i] = dm(h, fv[i]);
-    for (int i = 0; i < 4; ++i)
-      xt[i] = da(da(da(da(x[i], dm(b51, k1[i])), dm(b52, k2[i])), dm(b53, k3[i])), dm(b54, k4[i]));
-    fl_deriv<M>(f, t0, sign, xt, fv);
-    for (int i = 0; i < 4; ++i) k5[i] = dm(h, fv[i]);
-    for (int i = 0; i < 4; ++i)
-      xt[i] = da(da(da(da(da(x[i], dm(b61, k1[i])), dm(b62, k2[i])), dm(b63, k3[i])), dm(b64, k4[i])),
-                 dm(b65, k5[i]));
-    fl_deriv<M>(f, t0, sign, xt, fv);
-    for (int i = 0; i < 4; ++i) k6[i] = dm(h, fv[i]);
-    double r = 0.0;
-    for (int i = 0; i < 4; ++i) {
-      const double e = da(da(da(da(dm(r1, k1[i]), dm(r3, k3[i])), dm(r4, k4[i])), dm(r5, k5[i])), dm(r6, k6[i]));
-      const double ri = fabs(e) / h;
-      if (i == 0 || ri > r) r = ri;
+  constexpr double hmin = 1e-6;
+  constexpr double quarter = 0.4978;  // under 0.84^4: below quarter * tol the factor is above 1
+  const double tol = forward ? 1e-3 : 1e-4;  // fieldline.py:67 and :92
+  const int dirn = forward ? 1 : -1;
+  int idx = cap;  // slot of the start point
+  double x[3] = {X[0], X[1], X[2]}, u[3], mag, s = 0.0;
+  fl_unit<M>(f, t0, x, u, mag);
+  for (int guard = 0; guard < 4 * cap; ++guard) {
+    const int before = idx;
+    double t = 0.0, h = ds;
+    bool raised = false;
+    for (int inner = 0; inner < 100000 && t < ds; ++inner) {
+      if (da(t, h) > ds) h = da(ds, -t);
+      const double hs = forward ? h : -h;  // h b and h (-b) alike
+      double k1[3], k2[3], k3[3], k4[3], k5[3], k6[3], xt[3], v[3], m;
+#pragma unroll
+      for (int i = 0; i < 3; ++i) { k1[i] = dm(hs, u[i]); xt[i] = da(x[i], dm(b21, k1[i])); }
+      fl_unit<M>(f, t0, xt, v, m);
+#pragma unroll
+      for (int i = 0; i < 3; ++i) { k2[i] = dm(hs, v[i]); xt[i] = da(da(x[i], dm(b31, k1[i])), dm(b32, k2[i])); }
+      fl_unit<M>(f, t0, xt, v, m);
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        k3[i] = dm(hs, v[i]);
+        xt[i] = da(da(da(x[i], dm(b41, k1[i])), dm(b42, k2[i])), dm(b43, k3[i]));
+      }
+      fl_unit<M>(f, t0, xt, v, m);
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        k4[i] = dm(hs, v[i]);
+        xt[i] = da(da(da(da(x[i], dm(b51, k1[i])), dm(b52, k2[i])), dm(b53, k3[i])), dm(b54, k4[i]));
+      }
+      fl_unit<M>(f, t0, xt, v, m);
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        k5[i] = dm(hs, v[i]);
+        xt[i] = da(da(da(da(da(x[i], dm(b61, k1[i])), dm(b62, k2[i])), dm(b63, k3[i])), dm(b64, k4[i])),
+                   dm(b65, k5[i]));
+      }
+      fl_unit<M>(f, t0, xt, v, m);
+      double e = 0.0;  // max_i |sum_j r_j k_j|
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        k6[i] = dm(hs, v[i]);
+        e = fmax(e, fabs(da(da(da(da(dm(r1, k1[i]), dm(r3, k3[i])), dm(r4, k4[i])), dm(r5, k5[i])), dm(r6, k6[i]))));
+      }
+      const double r = e / h;
+      if (r <= tol) {
+        t = da(t, h);
+        s = da(da(da(da(s, dm(c1, hs)), dm(c3, hs)), dm(c4, hs)), dm(c5, hs));
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+          x[i] = da(da(da(da(x[i], dm(c1, k1[i])), dm(c3, k3[i])), dm(c4, k4[i])), dm(c5, k5[i]));
+        idx += dirn;
+        if (idx < 0 || idx > 2 * cap - 1) { overflow = true; return before; }
+        fl_unit<M>(f, t0, x, u, mag);
+        if (!isfinite(mag)) { overflow = true; return before; }
+        S[idx] = s;
+        Bs[idx] = mag;
+      }
+      if (h != ds || r > quarter * tol) h = dm(h, fmin(fmax(dm(0.84, pow(tol / r, 0.25)), 0.1), 4.0));
+      if (h > ds) h = ds;
+      else if (h < hmin) { raised = true; break; }
     }
-    if (r <= tol) {
-      t = da(t, h);
-      for (int i = 0; i < 4; ++i) x[i] = da(da(da(da(x[i], dm(c1, k1[i])), dm(c3, k3[i])), dm(c4, k4[i])), dm(c5, k5[i]));
-      idx += dirn;
-      if (idx < lo || idx > hi) { overflow = true; return false; }
-      S[idx] = x[0];
-      Bs[idx] = fl_magB<M>(f, t0, x[1], x[2], x[3]);
-    }
-    h = dm(h, fmin(fmax(dm(0.84, pow(tol / r, 0.25)), 0.1), 4.0));
-    if (h > hmax) h = hmax;
-    else if (h < hmin) return false;
+    if (raised) return before;
+    if (mag > Bm) break;
   }
-  return true;
+  return idx;
 }
 
 // ---------------------------------------------------------------- quadratic spline
@@ -166,8 +197,9 @@ struct DSpline2 {
       }
     }
   }
-  __device__ __forceinline__ double operator()(double v) const {
-    const int l = find(v);
+  __device__ __forceinline__ double operator()(double v) const { return on(v, find(v)); }
+  // the value at v on panel l
+  __device__ __forceinline__ double on(double v, int l) const {
     double h[3];
     basis(v, l, h);
     double y = 0.0;
@@ -182,7 +214,7 @@ static __device__ __noinline__ void spline2_solve(const double* x, double* yc, d
   DSpline2 sp{x, yc, n};
   // forward elimination row by row (the lower entry is formed when the row is built)
   for (int i = 0; i < n; ++i) {
-    const int l = sp.find(x[i]);
+    const int l = min(max(i + 1, 2), n - 1);  // the panel that holds x[i]
     double h[3];
     sp.basis(x[i], l, h);
     double lo = 0.0, d = 0.0, u = 0.0;
@@ -268,7 +300,7 @@ static __device__ __noinline__ double fl_brentq(const MirrorFn& f, double xa, do
 // same spline is integrated to convergence instead: s = c + h sin(theta)
 // removes the singularities and an 8-point Gauss-Legendre rule runs on every
 // panel between the images of the spline's knots.
-__device__ __forceinline__ void gauss_legendre8(double* x, double* w) {
+static __device__ __noinline__ void gauss_legendre8(double* x, double* w) {
   const int n = 8;
   for (int i = 0; i < n / 2; ++i) {
     double z = cos(kPi * (i + 0.75) / (n + 0.5)), pp = 0.0;
@@ -290,87 +322,196 @@ __device__ __forceinline__ void gauss_legendre8(double* x, double* w) {
   }
 }
 
-// INV: integrand 1/sqrt(1 - B/Bm) (half-bounce path); otherwise sqrt(1 - B/Bm)
+// inv: integrand 1/sqrt(1 - B/Bm) (half-bounce path); otherwise sqrt(1 - B/Bm)
 // (the second invariant I), which the substitution leaves smooth as well.
-template <bool INV = true>
-static __device__ __noinline__ double fl_bounce_integral(const DSpline2& sp, double sm1, double sm2, double Bm) {
+// Panel edges in theta: -pi/2, the knots j0 .. j1 inside (sm1, sm2), pi/2.
+struct FlPanels {
+  double c, h;
+  int j0, count;  // first knot inside; panels
+};
+__device__ __forceinline__ FlPanels fl_panels(const DSpline2& sp, double sm1, double sm2) {
+  FlPanels P{dm(0.5, da(sm1, sm2)), dm(0.5, da(sm2, -sm1)), 0, 1};
+  for (int j = 3; j < sp.n; ++j) {
+    const double tj = sp.knot(j);
+    if (!(tj > sm1 && tj < sm2)) continue;
+    if (P.count == 1) P.j0 = j;
+    ++P.count;
+  }
+  return P;
+}
+__device__ __forceinline__ double fl_panel_edge(const DSpline2& sp, const FlPanels& P, int q) {
+  if (q == 0) return -kPi / 2;
+  return q == P.count ? kPi / 2 : asin((sp.knot(P.j0 + q - 1) - P.c) / P.h);
+}
+// One panel between its edges ea, eb: 8 nodes gx, weights gw. The spline panel
+// is the knots' own (found by search only where no knot lies inside).
+static __device__ __noinline__ double fl_panel_sum(const DSpline2& sp, const FlPanels& P, int q, double ea, double eb,
+                                                   const double* gx, const double* gw, double Bm, bool inv) {
+  const double mid = dm(0.5, da(ea, eb)), half = dm(0.5, da(eb, -ea));
+  const int l = P.count == 1 ? sp.find(P.c) : P.j0 + q - 1;
+  double ps = 0.0;
+#pragma unroll 1
+  for (int k = 0; k < 8; ++k) {
+    const double th = da(mid, dm(half, gx[k]));
+    double sn, cs;
+    sincos(th, &sn, &cs);
+    const double arg = da(1.0, -(sp.on(da(P.c, dm(P.h, sn)), l) / Bm));
+    if (arg > 0.0) {
+      const double hc = dm(P.h, cs), root = sqrt(arg);
+      ps = da(ps, dm(gw[k], inv ? hc / root : dm(hc, root)));
+    }
+  }
+  return dm(half, ps);
+}
+static __device__ __noinline__ double fl_bounce_integral(const DSpline2& sp, double sm1, double sm2, double Bm,
+                                                         bool inv) {
   double gx[8], gw[8];
   gauss_legendre8(gx, gw);
-  const double c = dm(0.5, da(sm1, sm2)), h = dm(0.5, da(sm2, -sm1));
+  const FlPanels P = fl_panels(sp, sm1, sm2);
   double sum = 0.0, ea = -kPi / 2;
-  // panel edges: -pi/2, the knots inside (sm1, sm2) in order, pi/2
-  for (int j = 3; j <= sp.n; ++j) {
-    double eb;
-    if (j < sp.n) {
-      const double tj = sp.knot(j);
-      if (!(tj > sm1 && tj < sm2)) continue;
-      eb = asin((tj - c) / h);
-    } else {
-      eb = kPi / 2;
-    }
-    const double mid = dm(0.5, da(ea, eb)), half = dm(0.5, da(eb, -ea));
-    double ps = 0.0;
-    for (int k = 0; k < 8; ++k) {
-      const double th = da(mid, dm(half, gx[k]));
-      const double arg = da(1.0, -(sp(da(c, dm(h, sin(th)))) / Bm));
-      if (arg > 0.0) ps = da(ps, dm(gw[k], INV ? dm(h, cos(th)) / sqrt(arg) : dm(dm(h, cos(th)), sqrt(arg))));
-    }
-    sum = da(sum, dm(half, ps));
+  for (int q = 0; q < P.count; ++q) {
+    const double eb = fl_panel_edge(sp, P, q + 1);
+    sum = da(sum, fl_panel_sum(sp, P, q, ea, eb, gx, gw, Bm, inv));
     ea = eb;
   }
   return sum;
 }
 
-// ---------------------------------------------------------------- half-bounce path and bounce period
-// flutils.halfbouncepath (flutils.py:254-316) at position X, time t, mirror
-// field Bm. scratch: 4 * (2 * cap) doubles. Returns NaN where the trace
-// overflows the buffer or the result is not finite.
-// Fieldline(tpos, field, Bmax=Bm).trace() (fieldline.py:37-105) through X,
-// both directions joined in S, Bs [first, first + n0); false where the trace
-// overflows the buffer or the step is not finite.
-template <int M>
-__device__ bool fl_trace(const FieldP& f, double t, const double* X, double Bm, double flres, double* scratch,
-                         int cap, int& first, int& n0) {
-  double* S = scratch;                 // [2 cap] arc length of the joined curve
-  double* Bs = scratch + 2 * cap;      // [2 cap] |B|
-  const double ds = 1.0 / fl_curvature<M>(f, t, X) / flres;  // fieldline.py:31-35
-  if (!(ds > 0) || !isfinite(ds)) return false;
-  const int c0 = cap;  // slot of the start point
-  S[c0] = 0.0;
-  Bs[c0] = fl_magB<M>(f, t, X[0], X[1], X[2]);
-  int ifw = c0, ibw = c0;
-  bool overflow = false;
-  for (int dir = 0; dir < 2; ++dir) {
-    const double tol = dir == 0 ? 1e-3 : 1e-4;  // fieldline.py:67 and :92
-    const double sign = dir == 0 ? 1.0 : -1.0;
-    int& idx = dir == 0 ? ifw : ibw;
-    double x[4] = {0.0, X[0], X[1], X[2]};
-    for (int guard = 0; guard < 4 * cap; ++guard) {
-      // x holds the last point of this direction; where rkf raises, the
-      // reference keeps none of that call's points (fieldline.py:68-69)
-      const int before = idx;
-      if (!fl_rkf<M>(f, t, sign, x, ds, tol, ds, 1e-6, S, Bs, idx, dir == 0 ? 1 : -1, 0, 2 * cap - 1, overflow)) {
-        idx = before;
-        break;
-      }
-      if (Bs[idx] > Bm) break;
-    }
-    if (overflow) return false;
+// ---------------------------------------------------------------- the spline's integral in closed form
+// On one panel 1 - B/Bm is a quadratic q(u) = A0 + A1 u + A2 u^2, and with
+// ra = sqrt(q(a)), rb = sqrt(q(b)), D = b - a, w = D / (ra + rb), y = -A2 w^2,
+// f(y) = atan(sqrt y) / sqrt y (atanh for y < 0), g(y) = (1 - f(y)) / y:
+//   int_a^b du / sqrt(q) = 2 w f(y)
+//   int_a^b sqrt(q) du   = D (ra + rb) / 4 + w (2 (ra^2 + rb^2) - A2 D^2) / 4 - w^3 disc g(y) / 4
+// with disc = A1^2 - 4 A0 A2 (the elementary antiderivatives, rearranged so that
+// nothing cancels as A2 goes to 0). The mirror points, where ra or rb is 0, need
+// no care of their own.
+__device__ __forceinline__ void fl_atan_ratio(double y, double& fy, double& gy) {
+  if (fabs(y) < 0.04) {  // the alternating series of f; truncation under 1e-16
+    constexpr double c[11] = {1.0 / 3,  1.0 / 5,  1.0 / 7,  1.0 / 9,  1.0 / 11, 1.0 / 13,
+                              1.0 / 15, 1.0 / 17, 1.0 / 19, 1.0 / 21, 1.0 / 23};
+    double p = c[10];
+#pragma unroll
+    for (int k = 9; k >= 0; --k) p = fma(-y, p, c[k]);
+    gy = p;
+    fy = fma(-y, p, 1.0);
+  } else {
+    const double r = sqrt(fabs(y));
+    fy = (y > 0.0 ? atan(r) : atanh(r)) / r;
+    gy = (1.0 - fy) / y;
   }
-  first = ibw;
-  n0 = ifw - ibw + 1;  // joined curve: slots ibw .. ifw
-  return true;
 }
 
+// Interpolating quadratic spline of the samples yc at x (n >= 3; yc leaves as
+// the coefficients; rd, up: scratch) and the integral of 1/sqrt(1 - B/Bm) (inv)
+// or sqrt(1 - B/Bm) between its mirror points. The collocation matrix is
+// tridiagonal (x_i lies on panel i + 1): one forward sweep, and one backward
+// sweep that integrates each panel as its coefficients appear, the mirror
+// points being roots of the outermost panels' quadratics. ~85 FP64
+// instructions a point, where a binary search per value, Brent's method and 8
+// quadrature nodes a panel (a sine, a cosine and a spline value each) took
+// ~1,700. A line that is not one well between its outermost points (no sign
+// change there, or B > Bm in between) takes those routines, which skip the
+// stretches above Bm. 16,384 guiding centres at the bounce-period cadence,
+// advance(0.2), with the trace above: 56.0 ms before, 29.9 ms.
+static __device__ __noinline__ double fl_well(const double* x, double* yc, double* rd, double* up, int n, double Bm,
+                                              bool inv) {
+  bool bad = !(n >= 4 && yc[0] > Bm && yc[1] <= Bm && yc[n - 2] <= Bm && yc[n - 1] > Bm);
+  const double iBm = 1.0 / Bm, x0 = x[0], xl = x[n - 1];
+  rd[0] = 1.0;
+  up[0] = 0.0;
+  {
+    double T0 = x0, T1 = x0, T2 = n > 3 ? 0.5 * (x[1] + x[2]) : xl;
+    double r0 = 1.0 / (T2 - T0), cp = yc[0], rdp = 1.0, upp = 0.0;
+    for (int i = 1; i <= n - 2; ++i) {
+      const double T3 = i + 3 >= n ? xl : 0.5 * (x[i + 1] + x[i + 2]);
+      const double r1 = 1.0 / (T2 - T1), r2 = 1.0 / (T3 - T1);
+      const double a = T2 - x[i], c = x[i] - T1;
+      const double h0 = (a * r1) * (a * r0), h2 = (c * r1) * (c * r2);
+      const double m = h0 * rdp;
+      rdp = 1.0 / (1.0 - h0 - h2 - m * upp);
+      upp = h2;
+      cp = fma(-m, cp, yc[i]);
+      rd[i] = rdp; up[i] = upp; yc[i] = cp;
+      T0 = T1; T1 = T2; T2 = T3; r0 = r2;
+    }
+  }
+  double sum = 0.0, c2 = 0.0, c1 = yc[n - 1];
+  // knots T1, T2 of the panel in hand, walking down from panel n - 1
+  double T2 = xl, T1 = n > 3 ? 0.5 * (x[n - 3] + x[n - 2]) : x0, r2 = 1.0 / (T2 - T1), rhi = 0.0;
+  for (int i = n - 2; i >= 0; --i) {
+    const double c0 = i ? fma(-up[i], c1, yc[i]) * rd[i] : yc[0];
+    yc[i] = c0;
+    if (i <= n - 3 && !bad) {  // panel i + 2: coefficients c0, c1, c2
+      const bool left = i == 0, right = i == n - 3;
+      const double T0 = i <= 1 ? x0 : 0.5 * (x[i - 1] + x[i]);
+      const double D1 = T2 - T1, r1 = 1.0 / D1, r0 = 1.0 / (T2 - T0);
+      const double al = (c0 - c1) * iBm * r1 * r0, be = (c2 - c1) * iBm * r1 * r2;
+      const double C = fma(-c1, iBm, 1.0), A2 = -(al + be);
+      const double qa = fma(-al * D1, D1, C), qb = fma(-be * D1, D1, C);
+      double ua = 0.0, ub = D1, ra = 0.0, rb = rhi;
+      if (right) {  // q as a quadratic in the distance from the panel's end
+        const double B1 = 2.0 * be * D1, disc = fma(B1, B1, -4.0 * qb * A2);
+        bad = bad || !(qb < 0.0 && disc >= 0.0);
+        ub = D1 - (-2.0 * qb) / (B1 + sqrt(disc));
+        rb = 0.0;
+      }
+      if (left) {
+        const double B1 = 2.0 * al * D1, disc = fma(B1, B1, -4.0 * qa * A2);
+        bad = bad || !(qa < 0.0 && disc >= 0.0);
+        ua = (-2.0 * qa) / (B1 + sqrt(disc));
+      } else {
+        bad = bad || !(qa > 0.0);
+        ra = sqrt(qa);
+      }
+      const double D = ub - ua, mu = fma(A2, ua + ub, 2.0 * al * D1);
+      const double q2 = fma(ra, ra, rb * rb), AD = A2 * D;
+      const double disc = fma(mu, mu, fma(AD, AD, -2.0 * A2 * q2));
+      bad = bad || !(D > 0.0) || (A2 > 0.0 && disc >= 0.0 && fabs(mu) < AD);  // a stretch above Bm inside
+      const double w = D / (ra + rb);
+      double fy, gy;
+      fl_atan_ratio(-A2 * w * w, fy, gy);
+      if (inv) sum = fma(2.0 * w, fy, sum);
+      else sum += 0.25 * fma(D, ra + rb, w * (2.0 * q2 - AD * D - w * w * disc * gy));
+      rhi = ra;
+      T2 = T1; T1 = T0; r2 = r0;
+    }
+    c2 = c1;
+    c1 = c0;
+  }
+  if (!bad) return sum;
+  const DSpline2 sp{x, yc, n};
+  const MirrorFn g{sp, Bm};
+  const double sm1 = fl_brentq(g, x[0], x[1]);
+  const double sm2 = !inv && sp(x[n - 2]) == Bm ? x[n - 2] : fl_brentq(g, x[n - 2], x[n - 1]);
+  return fl_bounce_integral(sp, sm1, sm2, Bm, inv);
+}
+
+// ---------------------------------------------------------------- half-bounce path and bounce period
+// A thread's scratch: 4 * (2 * cap) doubles: arc length and |B| of the joined
+// curve, then (in place of |B|) the spline coefficients, and the solve's rows.
+//
+// Step of the trace through X (fieldline.py:31-35) and its start sample.
 template <int M>
-__device__ __noinline__ double fl_halfbouncepath(const FieldP& f, double t, const double* X, double Bm,
-                                                 double flres, double* scratch, int cap) {
-  double* S = scratch;                 // [2 cap] arc length of the joined curve
-  double* Bs = scratch + 2 * cap;      // [2 cap] |B|, then the spline coefficients
-  double* di = scratch + 4 * cap;      // [2 cap]
-  double* up = scratch + 6 * cap;      // [2 cap]
-  int first, n0;
-  if (!fl_trace<M>(f, t, X, Bm, flres, scratch, cap, first, n0)) return nan("");
+__device__ __forceinline__ double fl_start(const FieldP& f, double t, const double* X, double flres, double* scratch,
+                                           int cap) {
+  const double ds = 1.0 / fl_curvature<M>(f, t, X) / flres;
+  scratch[cap] = 0.0;
+  scratch[3 * cap] = fl_magB<M>(f, t, X[0], X[1], X[2]);
+  return ds;
+}
+
+// The samples that the integral is taken over: n from slot lo of the scratch, or
+// (n == 0) the answer itself.
+struct FlCut {
+  int lo, n;
+  double value;
+};
+// flutils.halfbouncepath (flutils.py:254-316) of the traced samples in slots
+// first .. first + n0 - 1, mirror field Bm.
+static __device__ __noinline__ FlCut fl_cut_path(const double* scratch, int cap, int first, int n0, double Bm) {
+  const double* S = scratch;
+  const double* Bs = scratch + 2 * cap;
   int fin = -1, lin = -1;
   for (int i = 0; i < n0; ++i)
     if (Bs[first + i] <= Bm) {
@@ -383,89 +524,117 @@ __device__ __noinline__ double fl_halfbouncepath(const FieldP& f, double t, cons
   const int lo = i1 < 0 ? 0 : i1, hi = i2 > n0 - 1 ? n0 - 1 : i2;
   const int n = hi - lo + 1;
   const double* s = S + first + lo;
-  double* b = Bs + first + lo;
+  const double* b = Bs + first + lo;
   if (n == 3) {  // equatorial (flutils.py:292-303)
     const double s12 = s[0] - s[1], s23 = s[1] - s[2], s13 = s[0] - s[2];
     const double B2s = 2 * da(da(dm(b[0], s23), -dm(b[1], s13)), dm(b[2], s12)) / dm(dm(s12, s13), s23);
-    return dm(kPi, sqrt(2 * Bm / B2s));
+    return FlCut{0, 0, dm(kPi, sqrt(2 * Bm / B2s))};
   }
-  if (n < 3) return nan("");
-  spline2_solve(s, b, di, up, n);
-  const DSpline2 sp{s, b, n};
-  const MirrorFn g{sp, Bm};
-  const double sm1 = fl_brentq(g, s[0], s[1]);
-  const double sm2 = fl_brentq(g, s[n - 2], s[n - 1]);
-  return fl_bounce_integral(sp, sm1, sm2, Bm);
+  if (n < 3) return FlCut{0, 0, nan("")};
+  return FlCut{first + lo, n, 0.0};
 }
 
-// flutils.eye (flutils.py:65-151), the second invariant I at X for mirror field
-// Bm, over the same trace: 0 where the line's minimum |B| exceeds Bm or equals
-// it (equatorial); the points with B < Bm plus one beyond each end; the
-// quadratic spline, brentq mirror points and the integral of sqrt(1 - B/Bm)
-// to convergence. The reference takes this spline branch at equatorial pitch
-// angles of 70 degrees and above; below, its Simpson branch calls an undefined
-// name and raises, and here the spline branch serves every pitch angle. NaN
-// where the trace overflows or the trimmed line fails the reference's assert.
-template <int M>
-__device__ __noinline__ double fl_eye(const FieldP& f, double t, const double* X, double Bm, double flres,
-                                     double* scratch, int cap) {
-  double* S = scratch;
-  double* Bs = scratch + 2 * cap;
-  double* di = scratch + 4 * cap;
-  double* up = scratch + 6 * cap;
-  int first, n0;
-  if (!fl_trace<M>(f, t, X, Bm, flres, scratch, cap, first, n0) || n0 < 1) return nan("");
+// flutils.eye (flutils.py:65-151) of the traced samples: 0 where the line's
+// minimum |B| exceeds Bm or equals it (equatorial); the points with B < Bm plus
+// one beyond each end. The reference takes this spline branch at equatorial
+// pitch angles of 70 degrees and above; below, its Simpson branch calls an
+// undefined name and raises, and here the spline branch serves every pitch
+// angle. NaN where the trimmed line fails the reference's assert.
+static __device__ __noinline__ FlCut fl_cut_eye(const double* scratch, int cap, int first, int n0, double Bm) {
+  const double* Bs = scratch + 2 * cap;
+  if (n0 < 1) return FlCut{0, 0, nan("")};
   double Bmin = Bs[first];
-  for (int i = 1; i < n0; ++i) Bmin = fmin(Bmin, Bs[first + i]);
-  if (Bmin > Bm) return 0.0;
-  if (fabs(Bmin - Bm) / Bm < 1e-12) return 0.0;
   int fin = -1, lin = -1;
-  for (int i = 0; i < n0; ++i)
-    if (Bs[first + i] < Bm) {
+  for (int i = 0; i < n0; ++i) {
+    const double v = Bs[first + i];
+    Bmin = fmin(Bmin, v);
+    if (v < Bm) {
       if (fin < 0) fin = i;
       lin = i;
     }
+  }
+  if (Bmin > Bm) return FlCut{0, 0, 0.0};
+  if (fabs(Bmin - Bm) / Bm < 1e-12) return FlCut{0, 0, 0.0};
   const int lo = fin - 1 < 0 ? 0 : fin - 1, hi = lin + 1 > n0 - 1 ? n0 - 1 : lin + 1;
   const int n = hi - lo + 1;
-  const double* s = S + first + lo;
-  double* b = Bs + first + lo;
-  if (!(n >= 3 && b[0] > Bm && b[1] < Bm && b[n - 2] < Bm && b[n - 1] > Bm)) return nan("");
-  spline2_solve(s, b, di, up, n);
-  const DSpline2 sp{s, b, n};
-  const MirrorFn g{sp, Bm};
-  const double sm1 = fl_brentq(g, s[0], s[1]);
-  const double sm2 = sp(s[n - 2]) == Bm ? s[n - 2] : fl_brentq(g, s[n - 2], s[n - 1]);
-  return fl_bounce_integral<false>(sp, sm1, sm2, Bm);
+  const double* b = Bs + first + lo;
+  if (!(n >= 3 && b[0] > Bm && b[1] < Bm && b[n - 2] < Bm && b[n - 1] > Bm)) return FlCut{0, 0, nan("")};
+  return FlCut{first + lo, n, 0.0};
+}
+
+__device__ __forceinline__ double fl_integral_of(double* scratch, int cap, const FlCut& cut, double Bm, bool inv) {
+  if (cut.n == 0) return cut.value;
+  return fl_well(scratch + cut.lo, scratch + 2 * cap + cut.lo, scratch + 4 * cap, scratch + 6 * cap, cut.n, Bm, inv);
+}
+
+// Both directions of the line through X by one thread; false where the trace
+// overflows the buffer or the step is not finite.
+template <int M>
+__device__ bool fl_trace(const FieldP& f, double t, const double* X, double Bm, double flres, double* scratch,
+                         int cap, int& first, int& n0) {
+  const double ds = fl_start<M>(f, t, X, flres, scratch, cap);
+  if (!(ds > 0) || !isfinite(ds)) return false;
+  bool overflow = false;
+  const int ifw = fl_trace_dir<M>(f, t, X, Bm, ds, true, scratch, scratch + 2 * cap, cap, overflow);
+  first = fl_trace_dir<M>(f, t, X, Bm, ds, false, scratch, scratch + 2 * cap, cap, overflow);
+  n0 = ifw - first + 1;
+  return !overflow;
+}
+
+template <int M>
+__device__ __noinline__ double fl_halfbouncepath(const FieldP& f, double t, const double* X, double Bm,
+                                                 double flres, double* scratch, int cap) {
+  int first, n0;
+  if (!fl_trace<M>(f, t, X, Bm, flres, scratch, cap, first, n0)) return nan("");
+  return fl_integral_of(scratch, cap, fl_cut_path(scratch, cap, first, n0, Bm), Bm, true);
+}
+
+template <int M>
+__device__ __noinline__ double fl_eye(const FieldP& f, double t, const double* X, double Bm, double flres,
+                                     double* scratch, int cap) {
+  int first, n0;
+  if (!fl_trace<M>(f, t, X, Bm, flres, scratch, cap, first, n0)) return nan("");
+  return fl_integral_of(scratch, cap, fl_cut_eye(scratch, cap, first, n0, Bm), Bm, false);
 }
 
 // flutils.gradI (flutils.py:153-229): central differences of I over d in the
 // two directions perpendicular to b built from (x, y, 0); one-sided where one
-// end has I = 0.
+// end has I = 0. v: the two directions.
 template <int M>
-__device__ void fl_gradI(const FieldP& f, double t, const double* X, double Bm, double d, double flres,
-                         double* scratch, int cap, double* out) {
+__device__ __forceinline__ void fl_gradI_axes(const FieldP& f, double t, const double* X, double v[2][3]) {
   const double sc = fmax(fabs(X[0]), fabs(X[1]));
-  double r[3] = {X[0] / sc, X[1] / sc, 0.0 / sc};
+  double* r = v[0];
+  r[0] = X[0] / sc; r[1] = X[1] / sc; r[2] = 0.0 / sc;
   double b[3], mag;
   unit_and_mag<M>(f, t, X[0], X[1], X[2], b, mag);
   const double rb = ndot3(r, b);
   for (int i = 0; i < 3; ++i) r[i] = da(r[i], -dm(rb, b[i]));
   const double rn = sqrt(ndot3(r, r));
   for (int i = 0; i < 3; ++i) r[i] = r[i] / rn;
-  const double v2[3] = {da(dm(b[1], r[2]), -dm(b[2], r[1])), da(dm(b[2], r[0]), -dm(b[0], r[2])),
-                        da(dm(b[0], r[1]), -dm(b[1], r[0]))};
-  double dI[2];
+  v[1][0] = da(dm(b[1], r[2]), -dm(b[2], r[1]));
+  v[1][1] = da(dm(b[2], r[0]), -dm(b[0], r[2]));
+  v[1][2] = da(dm(b[0], r[1]), -dm(b[1], r[0]));
+}
+// One difference quotient from I at X + d v, X - d v and X.
+__device__ __forceinline__ double fl_gradI_quotient(double Ip, double Im, double I0, double d) {
+  if (Ip == 0.0) return da(I0, -Im) / d;
+  if (Im == 0.0) return da(Ip, -I0) / d;
+  return da(Ip, -Im) / (2.0 * d);
+}
+template <int M>
+__device__ void fl_gradI(const FieldP& f, double t, const double* X, double Bm, double d, double flres,
+                         double* scratch, int cap, double* out) {
+  double v[2][3], dI[2];
+  fl_gradI_axes<M>(f, t, X, v);
   for (int k = 0; k < 2; ++k) {
-    const double* v = k == 0 ? r : v2;
-    const double xp[3] = {da(X[0], dm(d, v[0])), da(X[1], dm(d, v[1])), da(X[2], dm(d, v[2]))};
-    const double xm[3] = {da(X[0], -dm(d, v[0])), da(X[1], -dm(d, v[1])), da(X[2], -dm(d, v[2]))};
+    const double xp[3] = {da(X[0], dm(d, v[k][0])), da(X[1], dm(d, v[k][1])), da(X[2], dm(d, v[k][2]))};
+    const double xm[3] = {da(X[0], -dm(d, v[k][0])), da(X[1], -dm(d, v[k][1])), da(X[2], -dm(d, v[k][2]))};
     const double I1 = fl_eye<M>(f, t, xp, Bm, flres, scratch, cap);
     const double I2 = fl_eye<M>(f, t, xm, Bm, flres, scratch, cap);
-    if (I1 == 0.0) dI[k] = da(fl_eye<M>(f, t, X, Bm, flres, scratch, cap), -I2) / d;
-    else if (I2 == 0.0) dI[k] = da(I1, -fl_eye<M>(f, t, X, Bm, flres, scratch, cap)) / d;
-    else dI[k] = da(I1, -I2) / (2.0 * d);
+    const double I0 = I1 == 0.0 || I2 == 0.0 ? fl_eye<M>(f, t, X, Bm, flres, scratch, cap) : 0.0;
+    dI[k] = fl_gradI_quotient(I1, I2, I0, d);
   }
-  for (int i = 0; i < 3; ++i) out[i] = da(dm(dI[0], r[i]), dm(dI[1], v2[i]));
+  for (int i = 0; i < 3; ++i) out[i] = da(dm(dI[0], v[0][i]), dm(dI[1], v[1][i]));
 }
 
 // GuidingCenter.bounceperiod (GuidingCenter.py:593-606) at state (x, y, z, ppar).

@@ -124,8 +124,10 @@ cudaError_t bc_interval(const FieldP& f, const KParams& P, int64_t n, double* st
                         int32_t* status, int64_t* counters, int32_t* flag, double* scratch, long long stride,
                         int cap, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
-  k_bc_interval<kM><<<(unsigned)((n + 63) / 64), 64, 0, s>>>(f, P, n, st, cst, plan, d, j, rows, max_rows, nrows,
-                                                             status, counters, flag, scratch, stride, cap);
+  constexpr int kTeams = 64 / kBcTeam;  // per block
+  k_bc_interval<kM><<<(unsigned)((n + kTeams - 1) / kTeams), 64, 0, s>>>(f, P, n, st, cst, plan, d, j, rows, max_rows,
+                                                                         nrows, status, counters, flag, scratch,
+                                                                         stride, cap);
   return cudaGetLastError();
 }
 cudaError_t bc_eval(const FieldP& f, double flres, int what, int64_t n, const double* tpos, const double* Bm,

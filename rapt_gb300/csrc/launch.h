@@ -27,6 +27,9 @@ using BcIntervalFn = cudaError_t (*)(const FieldP& f, const KParams& P, int64_t 
                                      const double* plan, double d, int64_t j, double* rows, int max_rows,
                                      int32_t* nrows, int32_t* status, int64_t* counters, int32_t* flag,
                                      double* scratch, long long stride, int cap, cudaStream_t s);
+// trace slots (of stride doubles) that n tracers of one BcIntervalFn launch use: six
+// lines a tracer, tracers rounded up to whole blocks (bc_kernels.cuh)
+constexpr int64_t bc_trace_slots(int64_t n) { return 6 * ((n + 3) / 4 * 4); }
 using BcEvalFn = cudaError_t (*)(const FieldP& f, double flres, int what, int64_t n, const double* tpos,
                                  const double* Bm, double d, const double* cst, double* out, double* scratch,
                                  long long stride, int cap, cudaStream_t s);
