@@ -15,15 +15,32 @@
 
 namespace rapt {
 
+//
+// Besides B and E each model says what a stencil need not repeat:
+//  - kAxes: the coordinates (bit a) that B depends on. The samples x +- d e_a
+//    along another axis are the centre's value twice.
+//  - time(f, t): what B takes from the time, formed once per right-hand side
+//    and handed to Bt at every sample (a sine is as dear as a dipole sample).
+//  - kHasE: false where E is zero everywhere.
 template <int M>
 struct Field;
+
+template <bool HAS_E, int AXES>
+struct FieldTraits {
+  static constexpr bool kHasE = HAS_E;
+  static constexpr int kAxes = AXES;
+  __device__ __forceinline__ static double time(const FieldP&, double) { return 0.0; }
+};
 
 // EarthDipole, fields.py:282-317: B = -3 B0 Re^3 / r^5 (xz, yz, z^2 - r^2/3).
 // c0 = -3 B0 Re^3.
 template <>
-struct Field<RAPT_EARTH_DIPOLE> {
+struct Field<RAPT_EARTH_DIPOLE> : FieldTraits<false, 7> {
   static constexpr bool kStatic = true;
-  __device__ __forceinline__ static void B(const FieldP& f, double, double x, double y, double z, double* o) {
+  __device__ __forceinline__ static void B(const FieldP& f, double t, double x, double y, double z, double* o) {
+    Bt(f, 0.0, x, y, z, o);
+  }
+  __device__ __forceinline__ static void Bt(const FieldP& f, double, double x, double y, double z, double* o) {
     const double r2 = x * x + y * y + z * z;
     const double ri = rsqrt(r2);
     const double ri2 = ri * ri;
@@ -40,9 +57,12 @@ struct Field<RAPT_EARTH_DIPOLE> {
 // DoubleDipole, fields.py:319-362: two parallel dipoles, the image at x = distance
 // with relative strength k. c0 = -B0 Re^3, p[1] = distance, p[2] = k.
 template <>
-struct Field<RAPT_DOUBLE_DIPOLE> {
+struct Field<RAPT_DOUBLE_DIPOLE> : FieldTraits<false, 7> {
   static constexpr bool kStatic = true;
-  __device__ __forceinline__ static void B(const FieldP& f, double, double x, double y, double z, double* o) {
+  __device__ __forceinline__ static void B(const FieldP& f, double t, double x, double y, double z, double* o) {
+    Bt(f, 0.0, x, y, z, o);
+  }
+  __device__ __forceinline__ static void Bt(const FieldP& f, double, double x, double y, double z, double* o) {
     const double yz2 = y * y + z * z;
     const double r2a = x * x + yz2;
     const double ia = rsqrt(r2a);
@@ -66,9 +86,12 @@ struct Field<RAPT_DOUBLE_DIPOLE> {
 
 // UniformBz, fields.py:364-390.
 template <>
-struct Field<RAPT_UNIFORM_BZ> {
+struct Field<RAPT_UNIFORM_BZ> : FieldTraits<false, 0> {
   static constexpr bool kStatic = true;
-  __device__ __forceinline__ static void B(const FieldP& f, double, double, double, double, double* o) {
+  __device__ __forceinline__ static void B(const FieldP& f, double t, double x, double y, double z, double* o) {
+    Bt(f, 0.0, x, y, z, o);
+  }
+  __device__ __forceinline__ static void Bt(const FieldP& f, double, double, double, double, double* o) {
     o[0] = 0.0; o[1] = 0.0; o[2] = f.p[0];
   }
   __device__ __forceinline__ static void E(const FieldP&, double, double, double, double, double* o) {
@@ -78,9 +101,12 @@ struct Field<RAPT_UNIFORM_BZ> {
 
 // UniformCrossedEB, fields.py:392-427: E = (0, Ey, 0), B = (0, 0, Bz); static = False.
 template <>
-struct Field<RAPT_UNIFORM_CROSSED_EB> {
+struct Field<RAPT_UNIFORM_CROSSED_EB> : FieldTraits<true, 0> {
   static constexpr bool kStatic = false;
-  __device__ __forceinline__ static void B(const FieldP& f, double, double, double, double, double* o) {
+  __device__ __forceinline__ static void B(const FieldP& f, double t, double x, double y, double z, double* o) {
+    Bt(f, 0.0, x, y, z, o);
+  }
+  __device__ __forceinline__ static void Bt(const FieldP& f, double, double, double, double, double* o) {
     o[0] = 0.0; o[1] = 0.0; o[2] = f.p[1];
   }
   __device__ __forceinline__ static void E(const FieldP& f, double, double, double, double, double* o) {
@@ -91,13 +117,19 @@ struct Field<RAPT_UNIFORM_CROSSED_EB> {
 // VarEarthDipole, fields.py:429-470: dipole moment times (1 + amp sin(2 pi t / period)),
 // induced E ignored as in the reference. c0 = -B0 Re^3, c1 = 2 pi / period.
 template <>
-struct Field<RAPT_VAR_EARTH_DIPOLE> {
+struct Field<RAPT_VAR_EARTH_DIPOLE> : FieldTraits<false, 7> {
   static constexpr bool kStatic = false;
+  __device__ __forceinline__ static double time(const FieldP& f, double t) {
+    return f.c0 * (1.0 + f.p[0] * sin(f.c1 * t));
+  }
   __device__ __forceinline__ static void B(const FieldP& f, double t, double x, double y, double z, double* o) {
+    Bt(f, time(f, t), x, y, z, o);
+  }
+  __device__ __forceinline__ static void Bt(const FieldP&, double tm, double x, double y, double z, double* o) {
     const double r2 = x * x + y * y + z * z;
     const double ri = rsqrt(r2);
     const double ri2 = ri * ri;
-    const double s = f.c0 * (1.0 + f.p[0] * sin(f.c1 * t)) * (ri2 * ri2 * ri);
+    const double s = tm * (ri2 * ri2 * ri);
     o[0] = __dmul_rn(s, 3.0 * x * z);
     o[1] = __dmul_rn(s, 3.0 * y * z);
     o[2] = __dmul_rn(s, 2.0 * z * z - x * x - y * y);
@@ -110,9 +142,12 @@ struct Field<RAPT_VAR_EARTH_DIPOLE> {
 // Parabolic, fields.py:472-511: (B0 z/d, 0, Bn) for |z| <= 1, else
 // (sign(z) * 3.07e-5, 0, Bn) -- the reference uses the module-level B0 there.
 template <>
-struct Field<RAPT_PARABOLIC> {
+struct Field<RAPT_PARABOLIC> : FieldTraits<false, 4> {
   static constexpr bool kStatic = true;
-  __device__ __forceinline__ static void B(const FieldP& f, double, double, double, double z, double* o) {
+  __device__ __forceinline__ static void B(const FieldP& f, double t, double x, double y, double z, double* o) {
+    Bt(f, 0.0, x, y, z, o);
+  }
+  __device__ __forceinline__ static void Bt(const FieldP& f, double, double, double, double z, double* o) {
     if (fabs(z) <= 1.0) o[0] = f.p[0] * z / f.p[2];
     else o[0] = (z > 0.0) ? kB0 : ((z < 0.0) ? -kB0 : 0.0);
     o[1] = 0.0;
@@ -126,9 +161,12 @@ struct Field<RAPT_PARABOLIC> {
 // Harris current sheet with a normal component and a uniform dawn-dusk E:
 // B = (B0 tanh(z/L), 0, Bn), E = (0, Ey, 0). Not in the reference. c0 = 1/L.
 template <>
-struct Field<RAPT_HARRIS> {
+struct Field<RAPT_HARRIS> : FieldTraits<true, 4> {
   static constexpr bool kStatic = false;
-  __device__ __forceinline__ static void B(const FieldP& f, double, double, double, double z, double* o) {
+  __device__ __forceinline__ static void B(const FieldP& f, double t, double x, double y, double z, double* o) {
+    Bt(f, 0.0, x, y, z, o);
+  }
+  __device__ __forceinline__ static void Bt(const FieldP& f, double, double, double, double z, double* o) {
     o[0] = __dmul_rn(f.p[0], tanh(z * f.c0));
     o[1] = 0.0;
     o[2] = f.p[2];
@@ -142,13 +180,19 @@ struct Field<RAPT_HARRIS> {
 // E = -dB0/dt Re^3 (y, -x, 0) / r^3. Not in the reference.
 // c0 = -B0 Re^3, c1 = w = 2 pi / period, c2 = B0 amp w Re^3.
 template <>
-struct Field<RAPT_COMPRESSED_DIPOLE> {
+struct Field<RAPT_COMPRESSED_DIPOLE> : FieldTraits<true, 7> {
   static constexpr bool kStatic = false;
+  __device__ __forceinline__ static double time(const FieldP& f, double t) {
+    return f.c0 * (1.0 + f.p[1] * sin(f.c1 * t));
+  }
   __device__ __forceinline__ static void B(const FieldP& f, double t, double x, double y, double z, double* o) {
+    Bt(f, time(f, t), x, y, z, o);
+  }
+  __device__ __forceinline__ static void Bt(const FieldP&, double tm, double x, double y, double z, double* o) {
     const double r2 = x * x + y * y + z * z;
     const double ri = rsqrt(r2);
     const double ri2 = ri * ri;
-    const double s = f.c0 * (1.0 + f.p[1] * sin(f.c1 * t)) * (ri2 * ri2 * ri);
+    const double s = tm * (ri2 * ri2 * ri);
     o[0] = __dmul_rn(s, 3.0 * x * z);
     o[1] = __dmul_rn(s, 3.0 * y * z);
     o[2] = __dmul_rn(s, 2.0 * z * z - x * x - y * y);
@@ -320,9 +364,13 @@ static __device__ __noinline__ GridV6 grid_interp_BE(RAPT_GRID_ARGS, const doubl
 }
 
 template <>
-struct Field<RAPT_GRID> {
+struct Field<RAPT_GRID> : FieldTraits<true, 7> {
   static constexpr bool kStatic = false;  // the runtime flag f.is_static decides (field_static)
+  __device__ __forceinline__ static double time(const FieldP&, double t) { return t; }
   __device__ __forceinline__ static void B(const FieldP& f, double t, double x, double y, double z, double* o) {
+    Bt(f, time(f, t), x, y, z, o);
+  }
+  __device__ __forceinline__ static void Bt(const FieldP& f, double t, double x, double y, double z, double* o) {
     const GridV r = grid_interp(RAPT_GRID_PASS(f), f.gB, t, x, y, z);
     o[0] = r.a; o[1] = r.b; o[2] = r.c;
   }
@@ -470,37 +518,60 @@ __device__ __forceinline__ bool left_grid(double err) {
   return M == RAPT_GRID && isnan(err);
 }
 
-// Unit vector and magnitude of B at a point: one rsqrt.
+// Unit vector and magnitude of B at a point: one rsqrt. tm: Field<M>::time at the time.
+template <int M>
+__device__ __forceinline__ void unit_and_mag_t(const FieldP& f, double tm, double x, double y, double z, double* ub,
+                                               double& mag) {
+  double b[3];
+  Field<M>::Bt(f, tm, x, y, z, b);
+  unit_and_mag_of(b, ub, mag);
+}
 template <int M>
 __device__ __forceinline__ void unit_and_mag(const FieldP& f, double t, double x, double y, double z, double* ub,
                                              double& mag) {
-  double b[3];
-  Field<M>::B(f, t, x, y, z, b);
-  unit_and_mag_of(b, ub, mag);
+  unit_and_mag_t<M>(f, Field<M>::time(f, t), x, y, z, ub, mag);
 }
 
 // The reference's central-difference stencil (fields.py:111-131 gradB and
 // 176-200 curlb) evaluates B at the same six points x +- d e_i twice; here each
-// point is evaluated once and feeds both grad|B| and curl b.
+// point is evaluated once and feeds both grad|B| and curl b. Along an axis that
+// B does not depend on both samples are the centre's (cu, cm: its unit vector
+// and magnitude), whose differences are formed all the same: zero, or NaN where
+// the field is. In the Harris sheet that is two tanh samples instead of six.
 template <int M>
-__device__ __forceinline__ void stencil_gradB_curlb(const FieldP& f, double t, const double* X, double* gB,
-                                                    double* cb) {
+__device__ __forceinline__ void stencil_gradB_curlb(const FieldP& f, double tm, const double* X, const double* cu,
+                                                    double cm, double* gB, double* cb) {
   double c0 = 0.0, c1 = 0.0, c2 = 0.0;
   const double d = f.gradstep;
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
     double up[3], um[3], mp, mm;
-    double xp[3] = {X[0], X[1], X[2]}, xm[3] = {X[0], X[1], X[2]};
-    xp[a] = X[a] + d;
-    xm[a] = X[a] - d;
-    unit_and_mag<M>(f, t, xp[0], xp[1], xp[2], up, mp);
-    unit_and_mag<M>(f, t, xm[0], xm[1], xm[2], um, mm);
+    if (Field<M>::kAxes >> a & 1) {
+      double xp[3] = {X[0], X[1], X[2]}, xm[3] = {X[0], X[1], X[2]};
+      xp[a] = X[a] + d;
+      xm[a] = X[a] - d;
+      unit_and_mag_t<M>(f, tm, xp[0], xp[1], xp[2], up, mp);
+      unit_and_mag_t<M>(f, tm, xm[0], xm[1], xm[2], um, mm);
+    } else {
+      mp = mm = cm;
+#pragma unroll
+      for (int i = 0; i < 3; ++i) up[i] = um[i] = cu[i];
+    }
     gB[a] = (mp - mm) * f.inv2d;
     if (a == 0) { c1 -= (up[2] - um[2]); c2 += (up[1] - um[1]); }
     if (a == 1) { c0 += (up[2] - um[2]); c2 -= (up[0] - um[0]); }
     if (a == 2) { c0 -= (up[1] - um[1]); c1 += (up[0] - um[0]); }
   }
   cb[0] = c0 * f.inv2d; cb[1] = c1 * f.inv2d; cb[2] = c2 * f.inv2d;
+}
+// With the centre's sample of its own (single evaluations).
+template <int M>
+__device__ __forceinline__ void stencil_gradB_curlb(const FieldP& f, double t, const double* X, double* gB,
+                                                    double* cb) {
+  const double tm = Field<M>::time(f, t);
+  double cu[3] = {0.0, 0.0, 0.0}, cm = 0.0;
+  if (Field<M>::kAxes != 7) unit_and_mag_t<M>(f, tm, X[0], X[1], X[2], cu, cm);
+  stencil_gradB_curlb<M>(f, tm, X, cu, cm, gB, cb);
 }
 
 // db/dt by central differences in time (fields.py:225-245); zero when static.
@@ -524,24 +595,26 @@ __device__ __forceinline__ double dBdt(const FieldP& f, double t, const double* 
   return (m2 - m1) / f.timestep / 2.0;
 }
 
-// |B| / max|dB_i/dx_j| (fields.py:247-261).
+// |B| / max|dB_i/dx_j| (fields.py:247-261). An axis that B does not depend on
+// adds a zero (or a NaN, which fmax passes over) to the maximum.
 template <int M>
 __device__ __forceinline__ double lengthscale(const FieldP& f, double t, const double* X) {
   double mx = 0.0;
-  const double d = f.gradstep;
+  const double d = f.gradstep, tm = Field<M>::time(f, t);
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
+    if (!(Field<M>::kAxes >> a & 1)) continue;
     double xp[3] = {X[0], X[1], X[2]}, xm[3] = {X[0], X[1], X[2]};
     xp[a] = X[a] + d;
     xm[a] = X[a] - d;
     double bp[3], bm[3];
-    Field<M>::B(f, t, xp[0], xp[1], xp[2], bp);
-    Field<M>::B(f, t, xm[0], xm[1], xm[2], bm);
+    Field<M>::Bt(f, tm, xp[0], xp[1], xp[2], bp);
+    Field<M>::Bt(f, tm, xm[0], xm[1], xm[2], bm);
 #pragma unroll
     for (int i = 0; i < 3; ++i) mx = fmax(mx, fabs((bp[i] - bm[i]) * f.inv2d));
   }
   double b[3];
-  Field<M>::B(f, t, X[0], X[1], X[2], b);
+  Field<M>::Bt(f, tm, X[0], X[1], X[2], b);
   return sqrt(dot3(b, b)) / mx;
 }
 

@@ -22,9 +22,14 @@ struct ParticleRHS {
     o[1] = Y[4] * igm;
     o[2] = Y[5] * igm;
     const double qg = charge * igm;
-    o[3] = charge * E[0] + qg * (Y[4] * B[2] - Y[5] * B[1]);
-    o[4] = charge * E[1] + qg * (Y[5] * B[0] - Y[3] * B[2]);
-    o[5] = charge * E[2] + qg * (Y[3] * B[1] - Y[4] * B[0]);
+    o[3] = qg * (Y[4] * B[2] - Y[5] * B[1]);
+    o[4] = qg * (Y[5] * B[0] - Y[3] * B[2]);
+    o[5] = qg * (Y[3] * B[1] - Y[4] * B[0]);
+    if (Field<M>::kHasE) {
+      o[3] = charge * E[0] + qg * (Y[4] * B[2] - Y[5] * B[1]);
+      o[4] = charge * E[1] + qg * (Y[5] * B[0] - Y[3] * B[2]);
+      o[5] = charge * E[2] + qg * (Y[3] * B[1] - Y[4] * B[0]);
+    }
     if (eq) { o[2] = 0.0; o[5] = 0.0; }
   }
 };
@@ -47,6 +52,7 @@ struct GcRHS {
     const double ppar = Y[3];
     double ub[3], Bmag;
     double B[3], gB[3], cb[3], Eg[3], dbg[3];
+    const double tm = Field<M>::time(f, t);
     if constexpr (M == RAPT_GRID) {
       // B, E, the stencil and db/dt from one cell search (grid_gc_fields)
       const GridFields g = grid_gc_fields(RAPT_GRID_PASS(f), f.gB, eom == 0 ? f.gE : nullptr, t, Y[0], Y[1], Y[2],
@@ -54,7 +60,7 @@ struct GcRHS {
 #pragma unroll
       for (int k = 0; k < 3; ++k) { B[k] = g.B[k]; Eg[k] = g.E[k]; gB[k] = g.gB[k]; cb[k] = g.cb[k]; dbg[k] = g.db[k]; }
     } else {
-      Field<M>::B(f, t, Y[0], Y[1], Y[2], B);
+      Field<M>::Bt(f, tm, Y[0], Y[1], Y[2], B);
     }
     {
       const double b2 = dot3(B, B);
@@ -62,7 +68,7 @@ struct GcRHS {
       Bmag = b2 * ib;
       ub[0] = B[0] * ib; ub[1] = B[1] * ib; ub[2] = B[2] * ib;
     }
-    if constexpr (M != RAPT_GRID) stencil_gradB_curlb<M>(f, t, Y, gB, cb);
+    if constexpr (M != RAPT_GRID) stencil_gradB_curlb<M>(f, tm, Y, ub, Bmag, gB, cb);
     if (eom == 0) {
       const double pm = ppar * inv_mc;
       const double g2 = 1.0 + k_mu * Bmag + pm * pm;
@@ -81,7 +87,11 @@ struct GcRHS {
       const double mg = mu * rg;
       double Es[3];
 #pragma unroll
-      for (int i = 0; i < 3; ++i) Es[i] = E[i] - (ppar * db[i] + mg * gB[i]) * qinv;
+      for (int i = 0; i < 3; ++i) {
+        // the zero terms of static models and of models without E are left out
+        const double g = Field<M>::kStatic ? mg * gB[i] : ppar * db[i] + mg * gB[i];
+        Es[i] = Field<M>::kHasE ? E[i] - g * qinv : -(g * qinv);
+      }
       double Exb[3];
       cross3(Es, ub, Exb);
       const double a = ppar * rg * minv;
