@@ -730,6 +730,16 @@ static int advance_impl(Ctx* c, int kind, const double* delta, double delta_all,
     P.fl_scratch = c->fl_scratch;
   }
 
+  // Small ensembles: a few tracers a warp, spread over every sub-partition, the
+  // other lanes working in teams (the FP64 kernels; team_lanes in launch.h).
+  P.lanes_p = 32;
+  P.lanes_g = f32 || tab != 0 ? 32 : team_lanes(c->n, c->num_sms, c->field.model);
+  auto grid_of = [&](int bps, int lanes) {
+    const int64_t warps = (c->n + lanes - 1) / lanes, blocks = (warps * 32 + block - 1) / block;
+    return (int)std::min<int64_t>((int64_t)c->num_sms * bps, blocks);
+  };
+  const int grid_p = grid_of(bps_p, P.lanes_p), grid_g = grid_of(bps_g, P.lanes_g);
+
   CK(cudaEventRecord(c->ev0, s));
   if (resume) k_clear_rows_full<<<(unsigned)((N + 255) / 256), 256, 0, s>>>(E);
   else k_prepare<<<(unsigned)((N + 255) / 256), 256, 0, s>>>(E, d_delta, delta_all, kind);
@@ -750,16 +760,16 @@ static int advance_impl(Ctx* c, int kind, const double* delta, double delta_all,
   int round = 0;
   // one round: reset the queue heads and the pending count, run the particle
   // kernel and the guiding-centre kernel over the ensemble view Ev
-  auto enqueue_round = [&](const DevEnsemble& Ev, int grid_p, int grid_g, int blk) -> int {
+  auto enqueue_round = [&](const DevEnsemble& Ev, int gp, int gg, int blk) -> int {
     CK(cudaMemsetAsync(c->scratch, 0, 3 * sizeof(unsigned long long), s));  // queue[2], pending
     LaunchArgs a{Ev, P, c->scratch, 0, blk, s};
     if (kind != RAPT_KIND_GC) {
-      a.grid = grid_p;
+      a.grid = gp;
       CK(f32 ? T.particle32(a) : T.particle[tab](a));
       ++kl;
     }
     if (kind != RAPT_KIND_PARTICLE) {
-      a.grid = grid_g;
+      a.grid = gg;
       CK(dense ? T.gc_dense(a) : (tab != 0 ? T.gc[tab](a) : (f32 ? T.gc32_lrn[lrn](a) : T.gc_lrn[lrn](a))));
       ++kl;
     }
@@ -794,7 +804,7 @@ static int advance_impl(Ctx* c, int kind, const double* delta, double delta_all,
     int rc = RAPT_OK;
     const int64_t kl0 = kl;
     for (int r = 0; r < kGraphRounds && rc == RAPT_OK; ++r)
-      rc = enqueue_round(E, c->num_sms * bps_p, c->num_sms * bps_g, block);
+      rc = enqueue_round(E, grid_p, grid_g, block);
     if (rc == RAPT_OK) rc = read_pending();
     cudaError_t ec = cudaStreamEndCapture(s, &graph);
     if (rc) { if (graph) cudaGraphDestroy(graph); return rc; }
@@ -815,7 +825,7 @@ static int advance_impl(Ctx* c, int kind, const double* delta, double delta_all,
     cudaGraphExecDestroy(exec);
   } else {
     for (; round < max_rounds; ++round) {
-      int rc = enqueue_round(E, c->num_sms * bps_p, c->num_sms * bps_g, block);
+      int rc = enqueue_round(E, grid_p, grid_g, block);
       if (rc) return rc;
       ++launches;
       rc = read_pending();

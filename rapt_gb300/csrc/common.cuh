@@ -48,6 +48,7 @@ struct KParams {
   long long budget;        // RK step attempts per thread per launch
   int max_rows, max_sw;    // per-tracer output capacity
   int max_segments;        // Adaptive: cap on advance() calls per tracer
+  int lanes_p, lanes_g;    // tracers a warp of the particle / guiding-centre kernel holds at a time (0: 32)
   // step-size MLP (learned forms) and training-sample collection
   const uint32_t* mlp_w;   // packed BF16 weights
   const float* mlp_p;      // FP32 biases and normalisation

@@ -24,7 +24,7 @@ namespace rapt {
 constexpr int kDenseSpan = 16;
 
 template <int M>
-__global__ void __launch_bounds__(128) k_gc_dense(DevEnsemble E, KParams P, Scratch* S) {
+__global__ void __launch_bounds__(128) k_gc_dense(DevEnsemble E, const __grid_constant__ KParams P, Scratch* S) {
   int64_t idx = -1;
   bool exhausted = false;
   long long budget = P.budget;
@@ -102,72 +102,84 @@ __global__ void __launch_bounds__(128) k_gc_dense(DevEnsemble E, KParams P, Scra
   };
 
   for (;;) {
-    warp_refill(&S->queue[1], E, RAPT_MODE_GC, idx, exhausted, load);
+    warp_refill(&S->queue[1], E, RAPT_MODE_GC, P.lanes_g, idx, exhausted, load);
     if (__all_sync(kFull, idx < 0)) break;
-    if (idx < 0) continue;
 
     const GcRHS<M> rhs{P.f, charge, qinv, mu, minv, kmu, inv_mc, igv, gmv, gmv2, P.gc_eom, P.enforce_eq != 0};
 
     // ---- between steps: segment end, launch budget, row capacity
-    if (!(seg_ok && t_row < stop)) {
-      bool more = false;
-      if (P.kind == RAPT_KIND_ADAPTIVE && status != RAPT_ST_NONFINITE && status != RAPT_ST_BAD_INPUT &&
-          status != RAPT_ST_OUT_OF_GRID && status != RAPT_ST_RKF_HMIN && tcur < delta) {
-        if (nseg + 1 >= P.max_segments) {
-          status = RAPT_ST_ADAPTIVE_LIMIT;
-        } else {
-          more = true;
-          ++nseg;
-          begin_segment(delta - tcur);
+    if (idx >= 0) {
+      bool more = seg_ok && t_row < stop;
+      if (!more) {
+        if (P.kind == RAPT_KIND_ADAPTIVE && status != RAPT_ST_NONFINITE && status != RAPT_ST_BAD_INPUT &&
+            status != RAPT_ST_OUT_OF_GRID && status != RAPT_ST_RKF_HMIN && tcur < delta) {
+          if (nseg + 1 >= P.max_segments) {
+            status = RAPT_ST_ADAPTIVE_LIMIT;
+          } else {
+            more = true;
+            ++nseg;
+            begin_segment(delta - tcur);
+          }
+        }
+        if (!more) {
+          flags |= RAPT_FLAG_DONE;
+          st.done++;
+          if (status != RAPT_ST_OK) st.fail++;
+          store(idx, false);
+          idx = -1;
         }
       }
-      if (!more) {
-        flags |= RAPT_FLAG_DONE;
-        st.done++;
-        if (status != RAPT_ST_OK) st.fail++;
-        store(idx, false);
+      if (more && budget <= 0) {
+        store(idx, true);
         idx = -1;
-        continue;
+        exhausted = true;
+        st.pend++;
+        more = false;
+      }
+      if (more && nrows + kDenseSpan + 1 > P.max_rows) {  // room for the rows one step can cover
+        status = RAPT_ST_ROWS_FULL;
+        store(idx, true);
+        idx = -1;
       }
     }
-    if (budget <= 0) {
-      store(idx, true);
-      idx = -1;
-      exhausted = true;
-      st.pend++;
-      continue;
+    // ---- the first slope and HINIT (all 32 lanes go through the right-hand sides together)
+    const bool first = idx >= 0 && !k1_valid, probe = idx >= 0 && h == 0.0;
+    if (__any_sync(kFull, first)) {
+      GcWarpRHS<M>{rhs, first}(rt, y, k1);  // the FSAL slope at (rt, y): recomputed after a load, bit for bit
+      if (first) {
+        k1_valid = true;
+        st.rhs++;
+        if (h == 0.0) nfcn += 1;  // counted once per integration, not per launch
+      }
     }
-    if (nrows + kDenseSpan + 1 > P.max_rows) {  // room for the rows one step can cover
-      status = RAPT_ST_ROWS_FULL;
-      store(idx, true);
-      idx = -1;
-      continue;
-    }
-    if (!k1_valid) {  // the FSAL slope at (rt, y): recomputed after a load, bit for bit
-      rhs(rt, y, k1);
-      k1_valid = true;
-      st.rhs++;
-      if (h == 0.0) nfcn += 1;  // counted once per integration, not per launch
-    }
-    if (h == 0.0) {  // start of the segment's integration: HINIT once
-      h = hinit<4>(rhs, rt, y, k1, 1.0, 1.0 / 5.0, kDenseSpan * dt, P.rtol, P.atol);
-      st.rhs++;
-      nfcn += 1;
-      facold = 1e-4;
-      reject = false;
-      nst = 0;
+    if (__any_sync(kFull, probe)) {  // start of the segment's integration: HINIT once
+      const double h0 =
+          hinit<4>(GcWarpRHS<M>{rhs, probe}, rt, y, k1, 1.0, 1.0 / 5.0, kDenseSpan * dt, P.rtol, P.atol);
+      if (probe) {
+        h = h0;
+        st.rhs++;
+        nfcn += 1;
+        facold = 1e-4;
+        reject = false;
+        nst = 0;
+      }
     }
 
     // ---- one DOPRI5 attempt
     int fail = 0;
     bool row_end = false;  // the segment ended (last row, failure or a raised check)
-    if (nst > P.nsteps) fail = RAPT_ST_MAXSTEPS;
-    else if (0.1 * fabs(h) <= fabs(rt) * kUround) fail = RAPT_ST_HMIN;
-    else {
+    bool attempt = false;
+    if (idx >= 0) {
+      if (nst > P.nsteps) fail = RAPT_ST_MAXSTEPS;
+      else if (0.1 * fabs(h) <= fabs(rt) * kUround) fail = RAPT_ST_HMIN;
+      else attempt = true;
+    }
+    double y1[4], k7[4], dd[4], err;
+    dopri5_attempt_rolled<4, GcWarpRHS<M>, true>(GcWarpRHS<M>{rhs, attempt}, rt, y, k1, h, P.rtol, P.atol, y1, k7,
+                                                 err, dd);
+    if (attempt) {
       ++nst;
       --budget;
-      double y1[4], k7[4], dd[4], err;
-      dopri5_attempt_rolled<4, GcRHS<M>, true>(rhs, rt, y, k1, h, P.rtol, P.atol, y1, k7, err, dd);
       nfcn += 6;
       st.rhs += 6;
       const double fac11 = pow_fp64(err, expo1);
@@ -237,8 +249,7 @@ __global__ void __launch_bounds__(128) k_gc_dense(DevEnsemble E, KParams P, Scra
             }
           }
         }
-        if (idx < 0) continue;
-        if (!row_end) {
+        if (idx >= 0 && !row_end) {
 #pragma unroll
           for (int i = 0; i < 4; ++i) { k1[i] = k7[i]; y[i] = y1[i]; }
         }
@@ -250,7 +261,7 @@ __global__ void __launch_bounds__(128) k_gc_dense(DevEnsemble E, KParams P, Scra
         h = hnew;
       }
     }
-    if (fail) {
+    if (idx >= 0 && fail) {
       // the integration stops; as in the restarting kernel a failed interval
       // still leaves a row at the integrator's time (none outside a grid)
       seg_ok = false;
@@ -262,7 +273,7 @@ __global__ void __launch_bounds__(128) k_gc_dense(DevEnsemble E, KParams P, Scra
       }
       h = 0.0;
     }
-    if (seg_ok && !all_finite<4>(y)) { seg_ok = false; status = RAPT_ST_NONFINITE; h = 0.0; }
+    if (idx >= 0 && seg_ok && !all_finite<4>(y)) { seg_ok = false; status = RAPT_ST_NONFINITE; h = 0.0; }
   }
   st.flush(S);
 }

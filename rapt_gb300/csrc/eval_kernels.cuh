@@ -49,7 +49,7 @@ __global__ void k_field_eval(FieldP f, int what, int64_t n, const double* tpos, 
 
 // state[i] = (t, y0..y5, gm | mu); mode 0 particle (gm frozen), 1 GC.
 template <int M>
-__global__ void k_rhs_eval(KParams P, int mode, int64_t n, const double* state, const double* mass,
+__global__ void k_rhs_eval(const __grid_constant__ KParams P, int mode, int64_t n, const double* state, const double* mass,
                            const double* charge, const double* v, double* out) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;

@@ -10,6 +10,8 @@
 // fuse the last product into the difference, which then sees the unrounded
 // product and no longer takes the difference of two field values as the
 // reference's scheme does (a constant field would get a nonzero gradient).
+// The single-dipole models spell out every fused operation, so that a sample has the
+// same bits wherever it is inlined (one lane's stencil or a team's sample).
 #pragma once
 #include "common.cuh"
 
@@ -21,14 +23,17 @@ namespace rapt {
 //    along another axis are the centre's value twice.
 //  - time(f, t): what B takes from the time, formed once per right-hand side
 //    and handed to Bt at every sample (a sine is as dear as a dipole sample).
+//  - kTimeB: whether B depends on the time; where it does not, db/dt and d|B|/dt
+//    are differences of one sample with itself.
 //  - kHasE: false where E is zero everywhere.
 template <int M>
 struct Field;
 
-template <bool HAS_E, int AXES>
+template <bool HAS_E, int AXES, bool TIME_B = false>
 struct FieldTraits {
   static constexpr bool kHasE = HAS_E;
   static constexpr int kAxes = AXES;
+  static constexpr bool kTimeB = TIME_B;
   __device__ __forceinline__ static double time(const FieldP&, double) { return 0.0; }
 };
 
@@ -41,13 +46,14 @@ struct Field<RAPT_EARTH_DIPOLE> : FieldTraits<false, 7> {
     Bt(f, 0.0, x, y, z, o);
   }
   __device__ __forceinline__ static void Bt(const FieldP& f, double, double x, double y, double z, double* o) {
-    const double r2 = x * x + y * y + z * z;
+    const double zz = __dmul_rn(z, z);
+    const double r2 = __fma_rn(x, x, __fma_rn(y, y, zz));
     const double ri = rsqrt(r2);
     const double ri2 = ri * ri;
     const double s = f.c0 * (ri2 * ri2 * ri);
     o[0] = __dmul_rn(s, x * z);
     o[1] = __dmul_rn(s, y * z);
-    o[2] = __dmul_rn(s, z * z - r2 * (1.0 / 3.0));
+    o[2] = __dmul_rn(s, __fma_rn(r2, -1.0 / 3.0, zz));
   }
   __device__ __forceinline__ static void E(const FieldP&, double, double, double, double, double* o) {
     o[0] = o[1] = o[2] = 0.0;
@@ -117,22 +123,22 @@ struct Field<RAPT_UNIFORM_CROSSED_EB> : FieldTraits<true, 0> {
 // VarEarthDipole, fields.py:429-470: dipole moment times (1 + amp sin(2 pi t / period)),
 // induced E ignored as in the reference. c0 = -B0 Re^3, c1 = 2 pi / period.
 template <>
-struct Field<RAPT_VAR_EARTH_DIPOLE> : FieldTraits<false, 7> {
+struct Field<RAPT_VAR_EARTH_DIPOLE> : FieldTraits<false, 7, true> {
   static constexpr bool kStatic = false;
   __device__ __forceinline__ static double time(const FieldP& f, double t) {
-    return f.c0 * (1.0 + f.p[0] * sin(f.c1 * t));
+    return f.c0 * __fma_rn(f.p[0], sin(__dmul_rn(f.c1, t)), 1.0);
   }
   __device__ __forceinline__ static void B(const FieldP& f, double t, double x, double y, double z, double* o) {
     Bt(f, time(f, t), x, y, z, o);
   }
   __device__ __forceinline__ static void Bt(const FieldP&, double tm, double x, double y, double z, double* o) {
-    const double r2 = x * x + y * y + z * z;
-    const double ri = rsqrt(r2);
+    const double zz = __dmul_rn(z, z);
+    const double ri = rsqrt(__fma_rn(x, x, __fma_rn(y, y, zz)));
     const double ri2 = ri * ri;
     const double s = tm * (ri2 * ri2 * ri);
     o[0] = __dmul_rn(s, 3.0 * x * z);
     o[1] = __dmul_rn(s, 3.0 * y * z);
-    o[2] = __dmul_rn(s, 2.0 * z * z - x * x - y * y);
+    o[2] = __dmul_rn(s, __fma_rn(-x, x, __fma_rn(-y, y, 2.0 * zz)));
   }
   __device__ __forceinline__ static void E(const FieldP&, double, double, double, double, double* o) {
     o[0] = o[1] = o[2] = 0.0;
@@ -180,29 +186,28 @@ struct Field<RAPT_HARRIS> : FieldTraits<true, 4> {
 // E = -dB0/dt Re^3 (y, -x, 0) / r^3. Not in the reference.
 // c0 = -B0 Re^3, c1 = w = 2 pi / period, c2 = B0 amp w Re^3.
 template <>
-struct Field<RAPT_COMPRESSED_DIPOLE> : FieldTraits<true, 7> {
+struct Field<RAPT_COMPRESSED_DIPOLE> : FieldTraits<true, 7, true> {
   static constexpr bool kStatic = false;
   __device__ __forceinline__ static double time(const FieldP& f, double t) {
-    return f.c0 * (1.0 + f.p[1] * sin(f.c1 * t));
+    return f.c0 * __fma_rn(f.p[1], sin(__dmul_rn(f.c1, t)), 1.0);
   }
   __device__ __forceinline__ static void B(const FieldP& f, double t, double x, double y, double z, double* o) {
     Bt(f, time(f, t), x, y, z, o);
   }
   __device__ __forceinline__ static void Bt(const FieldP&, double tm, double x, double y, double z, double* o) {
-    const double r2 = x * x + y * y + z * z;
-    const double ri = rsqrt(r2);
+    const double zz = __dmul_rn(z, z);
+    const double ri = rsqrt(__fma_rn(x, x, __fma_rn(y, y, zz)));
     const double ri2 = ri * ri;
     const double s = tm * (ri2 * ri2 * ri);
     o[0] = __dmul_rn(s, 3.0 * x * z);
     o[1] = __dmul_rn(s, 3.0 * y * z);
-    o[2] = __dmul_rn(s, 2.0 * z * z - x * x - y * y);
+    o[2] = __dmul_rn(s, __fma_rn(-x, x, __fma_rn(-y, y, 2.0 * zz)));
   }
   __device__ __forceinline__ static void E(const FieldP& f, double t, double x, double y, double z, double* o) {
-    const double r2 = x * x + y * y + z * z;
-    const double ri = rsqrt(r2);
-    const double s = -f.c2 * cos(f.c1 * t) * (ri * ri * ri);
-    o[0] = s * y;
-    o[1] = -s * x;
+    const double ri = rsqrt(__fma_rn(x, x, __fma_rn(y, y, __dmul_rn(z, z))));
+    const double s = -f.c2 * cos(__dmul_rn(f.c1, t)) * (ri * ri * ri);
+    o[0] = __dmul_rn(s, y);
+    o[1] = __dmul_rn(-s, x);
     o[2] = 0.0;
   }
 };
@@ -364,7 +369,7 @@ static __device__ __noinline__ GridV6 grid_interp_BE(RAPT_GRID_ARGS, const doubl
 }
 
 template <>
-struct Field<RAPT_GRID> : FieldTraits<true, 7> {
+struct Field<RAPT_GRID> : FieldTraits<true, 7, true> {
   static constexpr bool kStatic = false;  // the runtime flag f.is_static decides (field_static)
   __device__ __forceinline__ static double time(const FieldP&, double t) { return t; }
   __device__ __forceinline__ static void B(const FieldP& f, double t, double x, double y, double z, double* o) {
@@ -518,6 +523,50 @@ __device__ __forceinline__ bool left_grid(double err) {
   return M == RAPT_GRID && isnan(err);
 }
 
+// B of a guiding-centre right-hand side's samples, bit for bit the same in one
+// lane's stencil and in a team's (rhs.cuh); fused_z: the samples x +- d e_z. For
+// the double dipole every rounding is spelled out, as nvcc contracted the stencil
+// when its six samples shared their squares (a square used by several of them is
+// rounded, and only z's own square at the z samples is fused into 2 z^2 - x^2):
+// the accept decisions of long runs follow these bits.
+template <int M>
+__device__ __forceinline__ void stencil_sample(const FieldP& f, double tm, double x, double y, double z, bool fused_z,
+                                               double* o) {
+  if constexpr (M == RAPT_DOUBLE_DIPOLE) {
+    const double xx = __dmul_rn(x, x), yy = __dmul_rn(y, y), z2 = 2.0 * z;
+    const double yz2 = __fma_rn(z, z, yy);
+    const double ia = rsqrt(__dadd_rn(xx, yz2));
+    const double ia2 = ia * ia;
+    const double sa = ia2 * ia2 * ia;
+    const double x2 = __dadd_rn(x, -f.p[1]);
+    const double xx2 = __dmul_rn(x2, x2);
+    const double ib = rsqrt(__dadd_rn(xx2, yz2));
+    const double ib2 = ib * ib;
+    const double sb = f.p[2] * (ib2 * ib2 * ib);
+    const double zz2 = __dmul_rn(z2, z), tz = 3.0 * z;
+    const double qa = fused_z ? __fma_rn(z2, z, -xx) : __dadd_rn(zz2, -xx);
+    const double qb = fused_z ? __fma_rn(z2, z, -xx2) : __dadd_rn(zz2, -xx2);
+    o[0] = __dmul_rn(f.c0, tz * __fma_rn(x, sa, __dmul_rn(x2, sb)));
+    o[1] = __dmul_rn(f.c0, tz * y * __dadd_rn(sa, sb));
+    o[2] = __dmul_rn(f.c0, __fma_rn(__dadd_rn(qa, -yy), sa, __dmul_rn(__dadd_rn(qb, -yy), sb)));
+  } else {
+    Field<M>::Bt(f, tm, x, y, z, o);
+  }
+}
+
+// |B| and b of a stencil sample (the same in a stencil and in a team).
+template <int M>
+__device__ __forceinline__ void sample_unit_and_mag(const double* b, double* ub, double& mag) {
+  if constexpr (M == RAPT_GRID) {
+    unit_and_mag_of(b, ub, mag);
+  } else {
+    const double b2 = __fma_rn(b[2], b[2], __fma_rn(b[1], b[1], __dmul_rn(b[0], b[0])));
+    const double ib = rsqrt(b2);
+    mag = __dmul_rn(b2, ib);
+    ub[0] = __dmul_rn(b[0], ib); ub[1] = __dmul_rn(b[1], ib); ub[2] = __dmul_rn(b[2], ib);
+  }
+}
+
 // Unit vector and magnitude of B at a point: one rsqrt. tm: Field<M>::time at the time.
 template <int M>
 __device__ __forceinline__ void unit_and_mag_t(const FieldP& f, double tm, double x, double y, double z, double* ub,
@@ -550,8 +599,11 @@ __device__ __forceinline__ void stencil_gradB_curlb(const FieldP& f, double tm, 
       double xp[3] = {X[0], X[1], X[2]}, xm[3] = {X[0], X[1], X[2]};
       xp[a] = X[a] + d;
       xm[a] = X[a] - d;
-      unit_and_mag_t<M>(f, tm, xp[0], xp[1], xp[2], up, mp);
-      unit_and_mag_t<M>(f, tm, xm[0], xm[1], xm[2], um, mm);
+      double b[3];
+      stencil_sample<M>(f, tm, xp[0], xp[1], xp[2], a == 2, b);
+      sample_unit_and_mag<M>(b, up, mp);
+      stencil_sample<M>(f, tm, xm[0], xm[1], xm[2], a == 2, b);
+      sample_unit_and_mag<M>(b, um, mm);
     } else {
       mp = mm = cm;
 #pragma unroll
@@ -579,8 +631,15 @@ template <int M>
 __device__ __forceinline__ void dbdt(const FieldP& f, double t, const double* X, double* o) {
   if (field_static<M>(f)) { o[0] = o[1] = o[2] = 0.0; return; }
   double u1[3], u2[3], m1, m2;
-  unit_and_mag<M>(f, t - f.timestep, X[0], X[1], X[2], u1, m1);
-  unit_and_mag<M>(f, t + f.timestep, X[0], X[1], X[2], u2, m2);
+  double b[3];
+  stencil_sample<M>(f, Field<M>::time(f, t - f.timestep), X[0], X[1], X[2], false, b);
+  sample_unit_and_mag<M>(b, u1, m1);
+  if (Field<M>::kTimeB) {
+    stencil_sample<M>(f, Field<M>::time(f, t + f.timestep), X[0], X[1], X[2], false, b);
+    sample_unit_and_mag<M>(b, u2, m2);
+  } else {
+    u2[0] = u1[0]; u2[1] = u1[1]; u2[2] = u1[2];
+  }
   const double s = 0.5 / f.timestep;
   o[0] = (u2[0] - u1[0]) * s; o[1] = (u2[1] - u1[1]) * s; o[2] = (u2[2] - u1[2]) * s;
 }
@@ -591,7 +650,8 @@ __device__ __forceinline__ double dBdt(const FieldP& f, double t, const double* 
   if (field_static<M>(f)) return 0.0;
   double u[3], m1, m2;
   unit_and_mag<M>(f, t - f.timestep, X[0], X[1], X[2], u, m1);
-  unit_and_mag<M>(f, t + f.timestep, X[0], X[1], X[2], u, m2);
+  if (Field<M>::kTimeB) unit_and_mag<M>(f, t + f.timestep, X[0], X[1], X[2], u, m2);
+  else m2 = m1;
   return (m2 - m1) / f.timestep / 2.0;
 }
 

@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(128, 2) k_particle32(DevEnsemble E, const __gr
   };
 
   for (;;) {
-    warp_refill(&S->queue[0], E, RAPT_MODE_PARTICLE, idx, exhausted, load);
+    warp_refill(&S->queue[0], E, RAPT_MODE_PARTICLE, 32, idx, exhausted, load);
     if (__all_sync(kFull, idx < 0)) break;
     if (idx < 0) continue;
 
@@ -334,7 +334,7 @@ __global__ void __launch_bounds__(128, 8) k_gc32(DevEnsemble E, const __grid_con
   };
 
   for (;;) {
-    warp_refill(&S->queue[1], E, RAPT_MODE_GC, idx, exhausted, load);
+    warp_refill(&S->queue[1], E, RAPT_MODE_GC, 32, idx, exhausted, load);
     if (__all_sync(kFull, idx < 0)) break;
     lr.infer(P, h);
     if (idx < 0) continue;

@@ -13,6 +13,21 @@ struct LaunchArgs {
   cudaStream_t stream;
 };
 
+// Tracers a warp of the guiding-centre kernels holds at a time (KParams::lanes_g).
+// With 32 a warp, an ensemble below 32 * 4 * SMs tracers leaves sub-partitions
+// idle while the busy ones issue whole right-hand sides. Spread over one warp a
+// sub-partition, and no more to a warp than a round of teams serves (rhs.cuh: 4
+// tracers, 2 where a team is 16 lanes), they take a quarter of the FP64
+// instructions a warp; up to three rounds' worth a sub-partition that is less of
+// the pipe than one full warp's right-hand sides.
+inline int team_lanes(int64_t n, int sms, int model) {
+  const int64_t warps = 4LL * sms, per = (n + warps - 1) / warps;
+  const bool timed = model == RAPT_VAR_EARTH_DIPOLE || model == RAPT_COMPRESSED_DIPOLE || model == RAPT_GRID;
+  const int most = timed ? 2 : 4;
+  if (per > 3 * most) return 32;
+  return (int)(per < 1 ? 1 : (per > most ? most : per));
+}
+
 using LaunchFn = cudaError_t (*)(const LaunchArgs&);
 using OccFn = int (*)(int block);
 using FieldEvalFn = cudaError_t (*)(const FieldP& f, int what, int64_t n, const double* tpos, double* out,

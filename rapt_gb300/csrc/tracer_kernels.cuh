@@ -226,12 +226,15 @@ struct LaneStats {
 // The queue runs over positions 0..n-1; E.order maps a position to a tracer
 // (longest expected work first, so that the lanes that finish last at the end
 // of a launch hold the shortest tracers). Must be called by all 32 lanes.
+// lanes > 0: only the first `lanes` lanes take tracers (small ensembles spread
+// over more warps, whose other lanes work in teams).
 template <class LoadFn>
-__device__ __forceinline__ void warp_refill(unsigned long long* queue, const DevEnsemble& E, int mode, int64_t& idx,
-                                            bool& exhausted, LoadFn&& load) {
+__device__ __forceinline__ void warp_refill(unsigned long long* queue, const DevEnsemble& E, int mode, int lanes,
+                                            int64_t& idx, bool& exhausted, LoadFn&& load) {
   const int lane = threadIdx.x & 31;
+  const bool takes = lanes <= 0 || lane < lanes;
   for (;;) {
-    const bool need = (idx < 0) && !exhausted;
+    const bool need = (idx < 0) && !exhausted && takes;
     const unsigned m = __ballot_sync(kFull, need);
     if (m == 0u) break;
     const int leader = __ffs(m) - 1;
@@ -331,7 +334,7 @@ __global__ void __launch_bounds__(128) k_particle(DevEnsemble E, KParams P, Scra
   };
 
   for (;;) {
-    warp_refill(&S->queue[0], E, RAPT_MODE_PARTICLE, idx, exhausted, load);
+    warp_refill(&S->queue[0], E, RAPT_MODE_PARTICLE, P.lanes_p, idx, exhausted, load);
     if (__all_sync(kFull, idx < 0)) break;
     if (idx < 0) continue;
 
@@ -538,7 +541,7 @@ __global__ void __launch_bounds__(128) k_particle(DevEnsemble E, KParams P, Scra
 // (a proposal replaces the controller's next step after an accepted step and
 // HINIT at the next interval; a rejected proposal falls back to the controller).
 template <int M, int TAB, int LRN = 0>
-__global__ void __launch_bounds__(128) k_gc(DevEnsemble E, KParams P, Scratch* S) {
+__global__ void __launch_bounds__(128) k_gc(DevEnsemble E, const __grid_constant__ KParams P, Scratch* S) {
   static_assert(LRN == 0 || TAB == 0, "the step learner drives the DOPRI5 controller");
   int64_t idx = -1;
   bool exhausted = false;
@@ -616,15 +619,16 @@ __global__ void __launch_bounds__(128) k_gc(DevEnsemble E, KParams P, Scratch* S
   };
 
   for (;;) {
-    warp_refill(&S->queue[1], E, RAPT_MODE_GC, idx, exhausted, load);
+    warp_refill(&S->queue[1], E, RAPT_MODE_GC, P.lanes_g, idx, exhausted, load);
     if (__all_sync(kFull, idx < 0)) break;
     lr.infer(P, h);
-    if (idx < 0) continue;
 
     const GcRHS<M> rhs{P.f, charge, qinv, mu, minv, kmu, inv_mc, igv, gmv, gmv2, P.gc_eom, P.enforce_eq != 0};
-    bool release = false;
 
-    if (!in_interval) {
+    // ---- between intervals: end of the advance() call, launch budget, row capacity
+    bool start = false;
+    if (idx >= 0 && !in_interval) {
+      start = true;
       if (!(seg_ok && rt < stop)) {
         bool more = false;
         if (P.kind == RAPT_KIND_ADAPTIVE && status != RAPT_ST_NONFINITE && status != RAPT_ST_BAD_INPUT &&
@@ -643,59 +647,75 @@ __global__ void __launch_bounds__(128) k_gc(DevEnsemble E, KParams P, Scratch* S
           if (status != RAPT_ST_OK) st.fail++;
           store(idx, false);
           idx = -1;
-          continue;
+          start = false;
         }
       }
-      if (budget <= 0) {
+      if (start && budget <= 0) {
         store(idx, true);
         idx = -1;
         exhausted = true;
         st.pend++;
-        continue;
+        start = false;
       }
-      if (nrows + 2 > P.max_rows) {
+      if (start && nrows + 2 > P.max_rows) {
         status = RAPT_ST_ROWS_FULL;
         store(idx, true);
         idx = -1;
-        continue;
+        start = false;
       }
+    }
+    // ---- start of one SciPy integrate(r.t + dt) call. All 32 lanes go through the
+    // right-hand sides of HINIT and of the attempt together (GcWarpRHS).
+    if (start) {
       xend = rt + dt;
       hmax = fabs(xend - rt);
       posneg = copysign(1.0, xend - rt);
       nst = 0;
       nacc_int = 0;
-      if (TAB == 0) {
-        if (!k1_valid) { rhs(rt, y, k1); k1_valid = true; st.rhs++; }
-        if (LRN == 2 && lr.have_prop) {
-          // learned first step of the interval instead of HINIT
-          h = posneg * fmin(fabs(h), hmax);
-          lr.have_prop = false;
-          nfcn += 1;
-        } else {
-          h = hinit<4>(rhs, rt, y, k1, posneg, 1.0 / 5.0, hmax, P.rtol, P.atol);
-          st.rhs++;
-          nfcn += 2;
-        }
+      in_interval = true;
+      if (TAB != 0) h = hmax;
+    }
+    if (TAB == 0 && __any_sync(kFull, start)) {
+      const bool first = start && !k1_valid;
+      GcWarpRHS<M>{rhs, first}(rt, y, k1);
+      if (first) { k1_valid = true; st.rhs++; }
+      const bool probe = start && !(LRN == 2 && lr.have_prop);
+      const double h0 = hinit<4>(GcWarpRHS<M>{rhs, probe}, rt, y, k1, posneg, 1.0 / 5.0, hmax, P.rtol, P.atol);
+      if (probe) {
+        h = h0;
+        st.rhs++;
+        nfcn += 2;
+      } else if (start) {
+        // learned first step of the interval instead of HINIT
+        h = posneg * fmin(fabs(h), hmax);
+        lr.have_prop = false;
+        nfcn += 1;
+      }
+      if (start) {
         facold = 1e-4;
         reject = false;
         last = false;
-      } else {
-        h = hmax;
       }
-      in_interval = true;
     }
 
+    // ---- one step attempt
     bool ended = false;
     int fail = 0;
     if (TAB == 0) {
-      if (nst > P.nsteps) { ended = true; fail = RAPT_ST_MAXSTEPS; }
-      else if (0.1 * fabs(h) <= fabs(rt) * kUround) { ended = true; fail = RAPT_ST_HMIN; }
-      else {
+      bool attempt = false;
+      if (idx >= 0) {
+        if (nst > P.nsteps) { ended = true; fail = RAPT_ST_MAXSTEPS; }
+        else if (0.1 * fabs(h) <= fabs(rt) * kUround) { ended = true; fail = RAPT_ST_HMIN; }
+        else attempt = true;
+      }
+      if (attempt) {
         if ((rt + 1.01 * h - xend) * posneg > 0.0) { lr.before_clip(h); h = xend - rt; last = true; }
         ++nst;
         --budget;
-        double y1[4], k7[4], err;
-        dopri5_attempt_rolled<4>(rhs, rt, y, k1, h, P.rtol, P.atol, y1, k7, err);
+      }
+      double y1[4], k7[4], err;
+      dopri5_attempt_rolled<4>(GcWarpRHS<M>{rhs, attempt}, rt, y, k1, h, P.rtol, P.atol, y1, k7, err);
+      if (attempt) {
         nfcn += 6;
         st.rhs += 6;
         lr.on_attempt(P, h, err, last);
@@ -726,9 +746,8 @@ __global__ void __launch_bounds__(128) k_gc(DevEnsemble E, KParams P, Scratch* S
             h = hnew;
           }
           lr.on_accept(P, idx, nacc, hstep, err, errprev, h, hmax, was_last, rej_before, nst - nacc_int <= 8,
-                     (flags & RAPT_FLAG_CHECK_ADIABATICITY) != 0,
-                     (float)y[0], (float)y[1],
-                       (float)y[2], (float)y[3], vs, interval_progress(xend, rt, hmax));
+                       (flags & RAPT_FLAG_CHECK_ADIABATICITY) != 0, (float)y[0], (float)y[1], (float)y[2],
+                       (float)y[3], vs, interval_progress(xend, rt, hmax));
         } else {
           hnew = h / fmin(facc1, fac11 / safe);
           reject = true;
@@ -737,7 +756,7 @@ __global__ void __launch_bounds__(128) k_gc(DevEnsemble E, KParams P, Scratch* S
           h = hnew;
         }
       }
-    } else {
+    } else if (idx >= 0) {
       if (!(rt < xend)) { ended = true; }
       else if (nst > 1000000) { ended = true; fail = RAPT_ST_MAXSTEPS; }
       else {
@@ -809,17 +828,13 @@ __global__ void __launch_bounds__(128) k_gc(DevEnsemble E, KParams P, Scratch* S
           E.status[idx] = status; E.flags[idx] = flags; E.nrows[idx] = nrows; E.nswitch[idx] = nswitch;
           E.nseg[idx] = nseg; E.seg_active[idx] = 0;
           idx = -1;
-          continue;
         } else {
           flags |= RAPT_FLAG_RAISED | RAPT_FLAG_DONE;
           st.done++;
+          store(idx, false);
+          idx = -1;
         }
-        release = true;
       }
-    }
-    if (release) {
-      store(idx, false);
-      idx = -1;
     }
   }
   st.flush(S);

@@ -1,0 +1,77 @@
+"""Guiding centres and particles worked on by teams of lanes (small ensembles, the
+end of a launch) end in the same bits as one tracer a lane: a tracer's result
+does not depend on how many others are advanced with it."""
+import numpy as np
+import pytest
+
+from rapt_gb300 import fields as F
+from rapt_gb300 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+BIG = 20011  # more than three rounds of four-tracer warps: one tracer a lane until the end of the launch
+
+
+def _grid_field():
+    return W.dipole_grid(41, 41, 21)
+
+
+def _static_grid_field():
+    g = W.dipole_grid(41, 41, 21)
+    g.static = True
+    return g
+
+
+MODELS = {"EarthDipole": F.EarthDipole, "DoubleDipole": F.DoubleDipole, "VarEarthDipole": F.VarEarthDipole,
+          "CompressedDipole": F.CompressedDipole, "Harris": F.Harris, "UniformCrossedEB": lambda: F.UniformCrossedEB(1e-4, 1e-7),
+          "Grid": _grid_field, "StaticGrid": _static_grid_field}
+
+
+def _run(field, kind, n, w, delta, **cfg):
+    from rapt_gb300 import Ensemble
+    ens = Ensemble(field, n, max_rows=48, max_switch=8)
+    ens.configure(rtol=1e-7, atol=1e-7, **cfg)
+    if kind == "gc":
+        ens.set_guiding_centers(w["pos"][:n], w["v"][:n], pa=w["pa"][:n], t0=0.5, mass=w["mass"][:n], charge=w["charge"][:n])
+    else:
+        ens.set_particles(w["pos"][:n], w["vel"][:n], 0.5, w["mass"][:n], w["charge"][:n])
+    ens.upload()
+    if kind == "adaptive":
+        ens.adaptive_init()
+    ens.advance(kind, delta)
+    h = ens.download()
+    rows, mode, nrows, _, _ = ens.rows()
+    k = min(n, 128)
+    return [h[a][..., :k].copy() for a in ("s", "t_row", "mu", "status", "mode", "naccept", "nreject", "nfcn")] + \
+        [nrows[:k].copy(), [rows[i, :nrows[i]].copy() for i in range(k)]]
+
+
+def _same(a, b, n):
+    for x, y in zip(a[:-1], b[:-1]):
+        assert np.array_equal(x[..., :n], y[..., :n], equal_nan=x.dtype.kind == "f")
+    for x, y in zip(a[-1][:n], b[-1][:n]):
+        assert np.array_equal(x, y, equal_nan=True)
+
+
+@pytest.mark.parametrize("model", list(MODELS))
+@pytest.mark.parametrize("eom", [0, 1, 2])
+def test_guiding_centre_teams(model, eom):
+    field = MODELS[model]()
+    w = W.config2(BIG, seed=5)
+    if model in ("Harris", "UniformCrossedEB"):
+        w = dict(w, mass=np.full(BIG, W.m_pr), charge=np.full(BIG, W.e), v=np.linspace(3e5, 3e6, BIG),
+                 pos=W.config3(BIG, 2)["pos"])
+    delta = 0.02 if model in ("Grid", "StaticGrid") else 0.05
+    cfg = dict(gctimestep=0.01, gc_eom=eom)
+    big = _run(field, "gc", BIG, w, delta, **cfg)
+    for n in (1, 7, 128):
+        _same(_run(field, "gc", n, w, delta, **cfg), big, n)
+
+
+@pytest.mark.parametrize("model", ["DoubleDipole", "CompressedDipole"])
+def test_dense_output_teams(model):
+    w = W.config2(BIG, seed=6)
+    cfg = dict(gctimestep=0.01, dense_output=1)
+    big = _run(MODELS[model](), "gc", BIG, w, 0.1, **cfg)
+    for n in (1, 33, 128):
+        _same(_run(MODELS[model](), "gc", n, w, 0.1, **cfg), big, n)
