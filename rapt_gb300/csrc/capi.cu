@@ -37,6 +37,10 @@ struct Ctx {
   void* tmp = nullptr;
   size_t tmp_bytes = 0;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+  // Adaptive rounds: the particle kernel runs beside the guiding-centre kernel
+  cudaStream_t side = nullptr;
+  cudaEvent_t fork = nullptr, join = nullptr;
+  int8_t* mode0 = nullptr;  // modes at the start of a round (in block)
   ModelTable tab[RAPT_N_MODELS];
   // step-size MLP: one device block of parameters, Adam moments, gradient,
   // loss and packed weights; a separate sample buffer
@@ -96,7 +100,7 @@ size_t ensemble_bytes(int64_t n, int max_rows, int max_sw) {
   auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
   const size_t N = (size_t)n;
   size_t b = 0;
-  b += 2 * al(N);                                      // mode, seg_active
+  b += 3 * al(N);                                      // mode, mode0, seg_active
   b += al(N * max_rows) + al(N * max_sw);              // row_mode, sw_mode
   b += 5 * al(N * 4);                                  // status, flags, nrows, nswitch, nseg
   b += 22 * al(N * 8);                                 // doubles
@@ -275,7 +279,10 @@ int rapt_ctx_create(int device, void** out) {
   if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaMalloc(&c->scratch, sizeof(Scratch)) != cudaSuccess ||
       cudaMallocHost(&c->h_pending, sizeof(unsigned long long)) != cudaSuccess ||
-      cudaEventCreate(&c->ev0) != cudaSuccess || cudaEventCreate(&c->ev1) != cudaSuccess) {
+      cudaEventCreate(&c->ev0) != cudaSuccess || cudaEventCreate(&c->ev1) != cudaSuccess ||
+      cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaEventCreateWithFlags(&c->fork, cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&c->join, cudaEventDisableTiming) != cudaSuccess) {
     delete c;
     return RAPT_ERR_CUDA;
   }
@@ -310,6 +317,9 @@ void rapt_ctx_destroy(void* ctx) {
   cudaFreeHost(c->h_pending);
   if (c->ev0) cudaEventDestroy(c->ev0);
   if (c->ev1) cudaEventDestroy(c->ev1);
+  if (c->fork) cudaEventDestroy(c->fork);
+  if (c->join) cudaEventDestroy(c->join);
+  if (c->side) cudaStreamDestroy(c->side);
   if (c->stream) cudaStreamDestroy(c->stream);
   delete c;
 }
@@ -477,6 +487,8 @@ int rapt_ensemble_alloc(void* ctx, int64_t n, int32_t max_rows, int32_t max_swit
   const size_t N = (size_t)n;
   E.n = n;
   E.mode = carve<int8_t>(p, N);
+  c->mode0 = carve<int8_t>(p, N);
+  E.mode0 = c->mode0;
   E.seg_active = carve<int8_t>(p, N);
   E.row_mode = carve<int8_t>(p, N * max_rows);
   E.sw_mode = carve<int8_t>(p, N * max_switch);
@@ -614,7 +626,7 @@ static int advance_impl(Ctx* c, int kind, const double* delta, double delta_all,
 static DevEnsemble ensemble_view(const DevEnsemble& E, int64_t k, int max_rows, int max_sw) {
   DevEnsemble V = E;
   V.n = 1;
-  V.mode += k; V.status += k; V.flags += k; V.t_int += k; V.t_row += k; V.tcur += k;
+  V.mode += k; V.mode0 += k; V.status += k; V.flags += k; V.t_int += k; V.t_row += k; V.tcur += k;
   for (int i = 0; i < 6; ++i) V.s[i] += k;
   V.mu += k; V.v += k; V.mass += k; V.charge += k;
   V.naccept += k; V.nreject += k; V.nfcn += k; V.nswitch += k;
@@ -738,7 +750,10 @@ static int advance_impl(Ctx* c, int kind, const double* delta, double delta_all,
     const int64_t warps = (c->n + lanes - 1) / lanes, blocks = (warps * 32 + block - 1) / block;
     return (int)std::min<int64_t>((int64_t)c->num_sms * bps, blocks);
   };
-  const int grid_p = grid_of(bps_p, P.lanes_p), grid_g = grid_of(bps_g, P.lanes_g);
+  // an Adaptive round's two kernels run side by side: each takes half of the SMs' blocks
+  const bool both = kind == RAPT_KIND_ADAPTIVE;
+  const int grid_p = grid_of(both ? (bps_p + 1) / 2 : bps_p, P.lanes_p);
+  const int grid_g = grid_of(both ? (bps_g + 1) / 2 : bps_g, P.lanes_g);
 
   CK(cudaEventRecord(c->ev0, s));
   if (resume) k_clear_rows_full<<<(unsigned)((N + 255) / 256), 256, 0, s>>>(E);
@@ -758,11 +773,23 @@ static int advance_impl(Ctx* c, int kind, const double* delta, double delta_all,
   int64_t launches = 0, kl = 1;
   const int max_rounds = 1000000;
   int round = 0;
-  // one round: reset the queue heads and the pending count, run the particle
-  // kernel and the guiding-centre kernel over the ensemble view Ev
+  // one round over the ensemble view Ev: reset the queue heads and the pending
+  // count, note the modes, and run the particle kernel and the guiding-centre
+  // kernel. In an Adaptive round they run side by side, each on the tracers that
+  // were of its mode at the start (a tracer that switches waits for the next
+  // round): both end in a tail of a few long tracers, which then overlap instead
+  // of following one another. 3,001 Adaptive tracers in the breathing dipole:
+  // 30.0 ms one after the other, 16.3 ms side by side (32,768 in the Harris sheet
+  // 105 ms either way: twice the rounds of half the length).
   auto enqueue_round = [&](const DevEnsemble& Ev, int gp, int gg, int blk) -> int {
     CK(cudaMemsetAsync(c->scratch, 0, 3 * sizeof(unsigned long long), s));  // queue[2], pending
+    CK(cudaMemcpyAsync(const_cast<int8_t*>(Ev.mode0), Ev.mode, (size_t)Ev.n, cudaMemcpyDeviceToDevice, s));
     LaunchArgs a{Ev, P, c->scratch, 0, blk, s};
+    if (both) {
+      CK(cudaEventRecord(c->fork, s));
+      CK(cudaStreamWaitEvent(c->side, c->fork, 0));
+      a.stream = c->side;
+    }
     if (kind != RAPT_KIND_GC) {
       a.grid = gp;
       CK(f32 ? T.particle32(a) : T.particle[tab](a));
@@ -770,8 +797,13 @@ static int advance_impl(Ctx* c, int kind, const double* delta, double delta_all,
     }
     if (kind != RAPT_KIND_PARTICLE) {
       a.grid = gg;
+      a.stream = s;
       CK(dense ? T.gc_dense(a) : (tab != 0 ? T.gc[tab](a) : (f32 ? T.gc32_lrn[lrn](a) : T.gc_lrn[lrn](a))));
       ++kl;
+    }
+    if (both) {
+      CK(cudaEventRecord(c->join, c->side));
+      CK(cudaStreamWaitEvent(s, c->join, 0));
     }
     return RAPT_OK;
   };

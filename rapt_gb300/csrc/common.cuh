@@ -70,6 +70,7 @@ struct KParams {
 struct DevEnsemble {
   int64_t n;
   int8_t* mode;
+  const int8_t* mode0;  // the modes at the start of a round: which kernel works on a tracer in it
   int32_t* status;
   int32_t* flags;
   double* t_int;     // integrator time r.t

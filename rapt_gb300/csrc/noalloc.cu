@@ -229,6 +229,7 @@ extern "C" int rapt_gc_advance_noalloc(int device, int model, const double* para
   E.nseg = ip + 2 * istride;
   int8_t* bp = reinterpret_cast<int8_t*>(base + kOffB);
   E.mode = bp;
+  E.mode0 = bp;
   E.seg_active = bp + al256(kMax);
   E.t_row = st->t;
   E.s[0] = st->x; E.s[1] = st->y; E.s[2] = st->z; E.s[3] = st->ppar;

@@ -222,7 +222,8 @@ struct LaneStats {
 };
 
 // Warp-wide refill: every lane without a tracer takes the next queue index
-// until it holds a tracer of this kernel's mode or the queue is exhausted.
+// until it holds a tracer of this kernel's mode (as of the start of the round)
+// or the queue is exhausted.
 // The queue runs over positions 0..n-1; E.order maps a position to a tracer
 // (longest expected work first, so that the lanes that finish last at the end
 // of a launch hold the shortest tracers). Must be called by all 32 lanes.
@@ -247,7 +248,7 @@ __device__ __forceinline__ void warp_refill(unsigned long long* queue, const Dev
         exhausted = true;
       } else {
         const int64_t k = E.order ? (int64_t)E.order[q] : (int64_t)q;
-        if (E.mode[k] == mode && !(E.flags[k] & RAPT_FLAG_DONE) && E.status[k] != RAPT_ST_ROWS_FULL) {
+        if (E.mode0[k] == mode && !(E.flags[k] & RAPT_FLAG_DONE) && E.status[k] != RAPT_ST_ROWS_FULL) {
           idx = k;
           load(idx);
         }
