@@ -102,7 +102,7 @@ size_t ensemble_bytes(int64_t n, int max_rows, int max_sw) {
   size_t b = 0;
   b += 3 * al(N);                                      // mode, mode0, seg_active
   b += al(N * max_rows) + al(N * max_sw);              // row_mode, sw_mode
-  b += 5 * al(N * 4);                                  // status, flags, nrows, nswitch, nseg
+  b += 7 * al(N * 4);                                  // status, flags, nrows, nswitch, nseg, ring[2]
   b += 22 * al(N * 8);                                 // doubles
   b += al(N * max_rows * 7 * 8) + al(N * max_sw * 8);  // rows, sw_time
   b += 3 * al(N * 8);                                  // int64 counters
@@ -222,6 +222,17 @@ __global__ void k_prepare(DevEnsemble E, const double* delta, double delta_all, 
   E.nseg[k] = 0;
   E.status[k] = RAPT_ST_OK;
   E.t_int[k] = E.t_row[k];
+}
+
+// Start of a k_adaptive launch: the tracers still to be advanced, counted.
+__global__ void k_count_left(DevEnsemble E, Scratch* S) {
+  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const bool left = k < E.n && !(E.flags[k] & RAPT_FLAG_DONE) && E.status[k] != RAPT_ST_ROWS_FULL;
+  const unsigned long long c = (unsigned long long)__syncthreads_count(left);
+  if (threadIdx.x == 0 && c) {
+    atomicAdd(&S->pending, c);
+    atomicAdd(&S->remaining, c);
+  }
 }
 
 __global__ void k_fill_defaults(DevEnsemble E, int have_tint, int have_tcur) {
@@ -497,6 +508,7 @@ int rapt_ensemble_alloc(void* ctx, int64_t n, int32_t max_rows, int32_t max_swit
   E.nrows = carve<int32_t>(p, N);
   E.nswitch = carve<int32_t>(p, N);
   E.nseg = carve<int32_t>(p, N);
+  for (int i = 0; i < 2; ++i) E.ring[i] = carve<int32_t>(p, N);
   E.t_int = carve<double>(p, N);
   E.t_row = carve<double>(p, N);
   E.tcur = carve<double>(p, N);
@@ -631,6 +643,7 @@ static DevEnsemble ensemble_view(const DevEnsemble& E, int64_t k, int max_rows, 
   V.mu += k; V.v += k; V.mass += k; V.charge += k;
   V.naccept += k; V.nreject += k; V.nfcn += k; V.nswitch += k;
   V.delta += k; V.seg_stop += k; V.seg_dt += k; V.seg_gm += k; V.seg_active += k; V.nseg += k;
+  V.ring[0] += k; V.ring[1] += k;
   V.carry_h += k; V.carry_fac += k; V.carry_nst += k;
   V.rows += (size_t)k * max_rows * 7;
   V.row_mode += (size_t)k * max_rows;
@@ -725,9 +738,17 @@ static int advance_impl(Ctx* c, int kind, const double* delta, double delta_all,
     bps_g = std::min(bps_g, c->cfg.blocks_per_sm);
   }
   if (bps_p < 1 || bps_g < 1) return fail(c, RAPT_ERR_CUDA, "kernel does not fit on an SM");
+  // Adaptive in the plain form: one grid for both modes, with hand-over (k_adaptive);
+  // it needs a block of each mode on an SM
+  int bps_a = kind == RAPT_KIND_ADAPTIVE && form == RAPT_FORM_PLAIN && tab == 0 && !dense && lrn == 0 &&
+                      !c->cfg.per_tracer_launches
+                  ? T.occ_adaptive(block)
+                  : 0;
+  if (c->cfg.blocks_per_sm > 0) bps_a = std::min(bps_a, 2 * c->cfg.blocks_per_sm);
   if (kind != RAPT_KIND_PARTICLE && c->cfg.gctimestep == 0) {
-    // bounce-period cadence: one field-line scratch slot per guiding-centre thread
-    const size_t threads = c->cfg.per_tracer_launches ? 32 : (size_t)c->num_sms * bps_g * block;
+    // bounce-period cadence: one field-line scratch slot per thread of a grid
+    const size_t threads =
+        c->cfg.per_tracer_launches ? 32 : (size_t)c->num_sms * (size_t)std::max(bps_g, bps_a) * block;
     const size_t bytes = threads * (size_t)P.fl_stride * sizeof(double);
     if (c->fl_bytes < bytes) {
       cudaFree(c->fl_scratch);
@@ -750,8 +771,10 @@ static int advance_impl(Ctx* c, int kind, const double* delta, double delta_all,
     const int64_t warps = (c->n + lanes - 1) / lanes, blocks = (warps * 32 + block - 1) / block;
     return (int)std::min<int64_t>((int64_t)c->num_sms * bps, blocks);
   };
-  // an Adaptive round's two kernels run side by side: each takes half of the SMs' blocks
-  const bool both = kind == RAPT_KIND_ADAPTIVE;
+  const bool hand = bps_a >= 2;
+  // otherwise an Adaptive round's two kernels run side by side: each takes half of the SMs' blocks
+  const bool both = kind == RAPT_KIND_ADAPTIVE && !hand;
+  const int grid_a = 2 * std::max(grid_of(bps_a / 2, P.lanes_p), grid_of(bps_a / 2, P.lanes_g));
   const int grid_p = grid_of(both ? (bps_p + 1) / 2 : bps_p, P.lanes_p);
   const int grid_g = grid_of(both ? (bps_g + 1) / 2 : bps_g, P.lanes_g);
 
@@ -778,13 +801,25 @@ static int advance_impl(Ctx* c, int kind, const double* delta, double delta_all,
   // kernel. In an Adaptive round they run side by side, each on the tracers that
   // were of its mode at the start (a tracer that switches waits for the next
   // round): both end in a tail of a few long tracers, which then overlap instead
-  // of following one another. 3,001 Adaptive tracers in the breathing dipole:
-  // 30.0 ms one after the other, 16.3 ms side by side (32,768 in the Harris sheet
-  // 105 ms either way: twice the rounds of half the length).
+  // of following one another. 3,001 Adaptive tracers in the breathing dipole, plain
+  // form: 30.0 ms one after the other, 16.3 ms side by side. The plain form now
+  // hands switched tracers over inside one launch (k_adaptive: 14.0 ms).
   auto enqueue_round = [&](const DevEnsemble& Ev, int gp, int gg, int blk) -> int {
-    CK(cudaMemsetAsync(c->scratch, 0, 3 * sizeof(unsigned long long), s));  // queue[2], pending
-    CK(cudaMemcpyAsync(const_cast<int8_t*>(Ev.mode0), Ev.mode, (size_t)Ev.n, cudaMemcpyDeviceToDevice, s));
+    CK(cudaMemsetAsync(c->scratch, 0, kRoundWords * sizeof(unsigned long long), s));
     LaunchArgs a{Ev, P, c->scratch, 0, blk, s};
+    if (kind == RAPT_KIND_ADAPTIVE)
+      CK(cudaMemcpyAsync(const_cast<int8_t*>(Ev.mode0), Ev.mode, (size_t)Ev.n, cudaMemcpyDeviceToDevice, s));
+    else
+      a.E.mode0 = Ev.mode;
+    if (hand) {
+      for (int i = 0; i < 2; ++i) CK(cudaMemsetAsync(Ev.ring[i], 0, (size_t)Ev.n * 4, s));
+      k_count_left<<<(unsigned)((Ev.n + 255) / 256), 256, 0, s>>>(Ev, c->scratch);
+      CK(cudaGetLastError());
+      a.grid = grid_a;
+      CK(T.adaptive(a));
+      kl += 2;
+      return RAPT_OK;
+    }
     if (both) {
       CK(cudaEventRecord(c->fork, s));
       CK(cudaStreamWaitEvent(c->side, c->fork, 0));

@@ -106,12 +106,20 @@ struct DevEnsemble {
   // work-queue order: queue position q hands out tracer order[q] (a permutation,
   // longest expected work first); null: index order
   const int32_t* order;
+  // hand-over rings of k_adaptive, n entries each ([mode]: tracers that switched to
+  // that mode, index + 1; 0: empty)
+  int32_t* ring[2];
 };
+constexpr int kRoundWords = 8;  // words of Scratch that are reset for every round
 
 // Scratch words used by the persistent kernels (one block of device memory).
 struct Scratch {
   unsigned long long queue[2];   // work-queue heads (particle kernel, GC kernel)
   unsigned long long pending;    // tracers left unfinished by the last launch pair
+  // k_adaptive: tracers not yet stopped in this launch, and the hand-over rings'
+  // read and write positions ([mode])
+  unsigned long long remaining;
+  unsigned long long ring_head[2], ring_tail[2];
   unsigned long long accepted, rejected, rhs, switches, done, failed;
 };
 

@@ -35,6 +35,15 @@ int occ_gc(int block) {
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_gc<kM, TAB>, block, 0);
   return nb;
 }
+cudaError_t launch_adaptive(const LaunchArgs& a) {
+  k_adaptive<kM><<<a.grid, a.block, 0, a.stream>>>(a.E, a.P, a.S);
+  return cudaGetLastError();
+}
+int occ_adaptive(int block) {
+  int nb = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_adaptive<kM>, block, 0);
+  return nb;
+}
 cudaError_t launch_gc_dense(const LaunchArgs& a) {
   k_gc_dense<kM><<<a.grid, a.block, 0, a.stream>>>(a.E, a.P, a.S);
   return cudaGetLastError();
@@ -174,6 +183,8 @@ void RAPT_CAT(register_model_, RAPT_MODEL)(ModelTable* t) {
   t->rhs_eval = rhs_eval;
   t->adaptive_init = adaptive_init;
   t->bounce_period = bounce_period;
+  t->adaptive = launch_adaptive;
+  t->occ_adaptive = occ_adaptive;
   t->gc_dense = launch_gc_dense;
   t->occ_gc_dense = occ_gc_dense;
   t->bc_start = bc_start;

@@ -257,6 +257,59 @@ __device__ __forceinline__ void warp_refill(unsigned long long* queue, const Dev
   }
 }
 
+// ---- hand-over between the two modes inside one launch (k_adaptive)
+// A tracer that switches is stored, fenced and put into the ring of its new mode;
+// a lane of that mode without a tracer takes it from there. A ring cannot run
+// over: it has n entries and a tracer is in at most one ring at a time. An entry
+// is published by its own store, so a taker sees only complete entries.
+__device__ __forceinline__ void hand_over(const DevEnsemble& E, Scratch* S, int mode, int64_t idx) {
+  __threadfence();
+  const unsigned long long at = atomicAdd(&S->ring_tail[mode], 1ull);
+  atomicExch(&E.ring[mode][at % (unsigned long long)E.n], (int32_t)idx + 1);
+}
+__device__ __forceinline__ int64_t take_over(const DevEnsemble& E, Scratch* S, int mode) {
+  for (int tries = 0; tries < 4; ++tries) {
+    const unsigned long long at = *(volatile unsigned long long*)&S->ring_head[mode];
+    int32_t* e = &E.ring[mode][at % (unsigned long long)E.n];
+    const int32_t v = *(volatile int32_t*)e;
+    if (v == 0) return -1;
+    if (atomicCAS(&S->ring_head[mode], at, at + 1) == at) {
+      atomicExch(e, 0);
+      __threadfence();
+      return (int64_t)v - 1;
+    }
+  }
+  return -1;
+}
+// A tracer has stopped for this launch; finished: it needs no further launch.
+__device__ __forceinline__ void retire(Scratch* S, bool finished) {
+  atomicAdd(&S->remaining, ~0ull);
+  if (finished) atomicAdd(&S->pending, ~0ull);
+}
+// Lanes that the work queue no longer feeds take switched tracers. A warp with no
+// tracer at all waits for one, until every tracer of the launch has stopped or
+// kPolls polls of about a microsecond have passed (what is left then goes to the
+// next launch); the waited-for lanes are blocks of the same launch.
+constexpr int kPolls = 1 << 18;
+template <class LoadFn>
+__device__ __forceinline__ void warp_take(const DevEnsemble& E, Scratch* S, int mode, int lanes, int64_t& idx,
+                                          bool exhausted, bool spent, LoadFn&& load) {
+  const int lane = threadIdx.x & 31;
+  const bool wants = exhausted && !spent && (lanes <= 0 || lane < lanes);
+  for (int poll = 0; poll < kPolls; ++poll) {
+    if (idx < 0 && wants) {
+      idx = take_over(E, S, mode);
+      if (idx >= 0) load(idx);
+    }
+    if (__any_sync(kFull, idx >= 0)) return;
+    if (!__any_sync(kFull, wants)) return;
+    unsigned long long left = 0;
+    if (lane == 0) left = *(volatile unsigned long long*)&S->remaining;
+    if (__shfl_sync(kFull, left, 0) == 0ull) return;
+    __nanosleep(1000);
+  }
+}
+
 __device__ __forceinline__ void put_row(const DevEnsemble& E, const KParams& P, int64_t idx, int& nrows, double t,
                                         const double* s, int ns, int mode) {
   double* r = E.rows + ((size_t)idx * (size_t)P.max_rows + (size_t)nrows) * 7;
@@ -269,10 +322,12 @@ __device__ __forceinline__ void put_row(const DevEnsemble& E, const KParams& P, 
 
 // ---------------------------------------------------------------- particle kernel
 // TAB 0: DOP853 with beta 0.1 (Particle.py:300); TAB 1: RKF45 (rkf.py).
-template <int M, int TAB>
-__global__ void __launch_bounds__(128) k_particle(DevEnsemble E, KParams P, Scratch* S) {
+// HAND: part of k_adaptive (switched tracers are handed over instead of left to
+// the next round).
+template <int M, int TAB, bool HAND>
+__device__ __forceinline__ void particle_body(const DevEnsemble& E, const KParams& P, Scratch* S) {
   int64_t idx = -1;
-  bool exhausted = false;
+  bool exhausted = false, spent = false;
   long long budget = P.budget;
   LaneStats st;
 
@@ -336,11 +391,12 @@ __global__ void __launch_bounds__(128) k_particle(DevEnsemble E, KParams P, Scra
 
   for (;;) {
     warp_refill(&S->queue[0], E, RAPT_MODE_PARTICLE, P.lanes_p, idx, exhausted, load);
+    if (HAND) warp_take(E, S, RAPT_MODE_PARTICLE, P.lanes_p, idx, exhausted, spent, load);
     if (__all_sync(kFull, idx < 0)) break;
     if (idx < 0) continue;
 
     const ParticleRHS<M> rhs{P.f, charge, mass2, igm, P.enforce_eq != 0};
-    bool release = false;
+    bool release = false, switched = false;
 
     if (!in_interval) {
       if (!(seg_ok && rt < stop)) {
@@ -361,6 +417,7 @@ __global__ void __launch_bounds__(128) k_particle(DevEnsemble E, KParams P, Scra
           st.done++;
           if (status != RAPT_ST_OK) st.fail++;
           store(idx, false);
+          if (HAND) retire(S, true);
           idx = -1;
           continue;
         }
@@ -368,13 +425,15 @@ __global__ void __launch_bounds__(128) k_particle(DevEnsemble E, KParams P, Scra
       if (budget <= 0) {
         store(idx, true);
         idx = -1;
-        exhausted = true;
-        st.pend++;
+        exhausted = spent = true;
+        if (HAND) retire(S, false);
+        else st.pend++;
         continue;
       }
       if (nrows + 2 > P.max_rows) {
         status = RAPT_ST_ROWS_FULL;
         store(idx, true);
+        if (HAND) retire(S, true);
         idx = -1;
         continue;
       }
@@ -514,7 +573,8 @@ __global__ void __launch_bounds__(128) k_particle(DevEnsemble E, KParams P, Scra
             const double first[6] = {g[0], g[1], g[2], g[3], mu, vs};
             put_row(E, P, idx, nrows, t_row, first, 6, RAPT_MODE_GC);
             st.sw++;
-            st.pend++;
+            switched = true;
+            if (!HAND) st.pend++;
           } else {
             status = RAPT_ST_GC_NOCONV;
             flags |= RAPT_FLAG_DONE;
@@ -530,10 +590,17 @@ __global__ void __launch_bounds__(128) k_particle(DevEnsemble E, KParams P, Scra
     }
     if (release) {
       store(idx, false);
+      if (HAND && switched) hand_over(E, S, RAPT_MODE_GC, idx);
+      else if (HAND) retire(S, true);
       idx = -1;
     }
   }
   st.flush(S);
+}
+
+template <int M, int TAB>
+__global__ void __launch_bounds__(128) k_particle(DevEnsemble E, const __grid_constant__ KParams P, Scratch* S) {
+  particle_body<M, TAB, false>(E, P, S);
 }
 
 // ---------------------------------------------------------------- guiding-centre kernel
@@ -541,11 +608,11 @@ __global__ void __launch_bounds__(128) k_particle(DevEnsemble E, KParams P, Scra
 // LRN (DOPRI5 only): 0 plain, 1 training-sample collection, 2 MLP step proposals
 // (a proposal replaces the controller's next step after an accepted step and
 // HINIT at the next interval; a rejected proposal falls back to the controller).
-template <int M, int TAB, int LRN = 0>
-__global__ void __launch_bounds__(128) k_gc(DevEnsemble E, const __grid_constant__ KParams P, Scratch* S) {
+template <int M, int TAB, int LRN, bool HAND>
+__device__ __forceinline__ void gc_body(const DevEnsemble& E, const KParams& P, Scratch* S) {
   static_assert(LRN == 0 || TAB == 0, "the step learner drives the DOPRI5 controller");
   int64_t idx = -1;
-  bool exhausted = false;
+  bool exhausted = false, spent = false;
   long long budget = P.budget;
   LaneStats st;
   StepLearner<LRN> lr;
@@ -621,6 +688,7 @@ __global__ void __launch_bounds__(128) k_gc(DevEnsemble E, const __grid_constant
 
   for (;;) {
     warp_refill(&S->queue[1], E, RAPT_MODE_GC, P.lanes_g, idx, exhausted, load);
+    if (HAND) warp_take(E, S, RAPT_MODE_GC, P.lanes_g, idx, exhausted, spent, load);
     if (__all_sync(kFull, idx < 0)) break;
     lr.infer(P, h);
 
@@ -647,6 +715,7 @@ __global__ void __launch_bounds__(128) k_gc(DevEnsemble E, const __grid_constant
           st.done++;
           if (status != RAPT_ST_OK) st.fail++;
           store(idx, false);
+          if (HAND) retire(S, true);
           idx = -1;
           start = false;
         }
@@ -654,13 +723,15 @@ __global__ void __launch_bounds__(128) k_gc(DevEnsemble E, const __grid_constant
       if (start && budget <= 0) {
         store(idx, true);
         idx = -1;
-        exhausted = true;
-        st.pend++;
+        exhausted = spent = true;
+        if (HAND) retire(S, false);
+        else st.pend++;
         start = false;
       }
       if (start && nrows + 2 > P.max_rows) {
         status = RAPT_ST_ROWS_FULL;
         store(idx, true);
+        if (HAND) retire(S, true);
         idx = -1;
         start = false;
       }
@@ -822,23 +893,45 @@ __global__ void __launch_bounds__(128) k_gc(DevEnsemble E, const __grid_constant
           nswitch = nsw;
           put_row(E, P, idx, nrows, t_row, s6, 6, RAPT_MODE_PARTICLE);
           st.sw++;
-          st.pend++;
+          if (!HAND) st.pend++;
           // store() below must not overwrite the particle state with the GC state
           E.t_int[idx] = rt; E.t_row[idx] = t_row; E.tcur[idx] = tcur;
           E.naccept[idx] = nacc; E.nreject[idx] = nrej; E.nfcn[idx] = nfcn;
           E.status[idx] = status; E.flags[idx] = flags; E.nrows[idx] = nrows; E.nswitch[idx] = nswitch;
           E.nseg[idx] = nseg; E.seg_active[idx] = 0;
+          if (HAND) hand_over(E, S, RAPT_MODE_PARTICLE, idx);
           idx = -1;
         } else {
           flags |= RAPT_FLAG_RAISED | RAPT_FLAG_DONE;
           st.done++;
           store(idx, false);
+          if (HAND) retire(S, true);
           idx = -1;
         }
       }
     }
   }
   st.flush(S);
+}
+
+template <int M, int TAB, int LRN = 0>
+__global__ void __launch_bounds__(128) k_gc(DevEnsemble E, const __grid_constant__ KParams P, Scratch* S) {
+  gc_body<M, TAB, LRN, false>(E, P, S);
+}
+
+// ---------------------------------------------------------------- Adaptive in one launch
+// Both modes in one grid (plain FP64 form): the first half of the blocks runs
+// particles, the second half guiding centres, and a tracer that switches is handed
+// to the other half at once. With a launch pair per round of switches, every round
+// ended in a tail of its longest segments (1.6-1.9 of 32 lanes active in most
+// rounds of the Harris sheet) while the tracers that had switched waited; here the
+// longest tracer alone sets the end. 32,768 Adaptive protons in the Harris sheet:
+// 105 ms in 15 rounds, 43.7 ms so; 3,001 tracers in the breathing dipole 16.3 and
+// 14.0 ms.
+template <int M>
+__global__ void __launch_bounds__(128) k_adaptive(DevEnsemble E, const __grid_constant__ KParams P, Scratch* S) {
+  if (blockIdx.x < gridDim.x / 2) particle_body<M, 0, true>(E, P, S);
+  else gc_body<M, 0, 0, true>(E, P, S);
 }
 
 }  // namespace rapt

@@ -75,3 +75,31 @@ def test_dense_output_teams(model):
     big = _run(MODELS[model](), "gc", BIG, w, 0.1, **cfg)
     for n in (1, 33, 128):
         _same(_run(MODELS[model](), "gc", n, w, 0.1, **cfg), big, n)
+
+
+@pytest.mark.parametrize("n", [1, 33, 2500])
+@pytest.mark.parametrize("cfg", [{}, {"max_steps_per_launch": 7}, {"use_graph": 1}, {"blocks_per_sm": 1, "threads_per_block": 64}])
+def test_adaptive_hand_over(n, cfg):
+    """Adaptive in one launch (switched tracers handed over on the device) against
+    one launch sequence per tracer: states, rows, switch logs and counters, with
+    step budgets that end launches in mid-flight, graph replay and other grids."""
+    from rapt_gb300 import Ensemble
+    w = W.config3(4096, seed=11)
+    d = 1.0 + 11.0 * np.random.default_rng(1).random(4096)
+    out = []
+    k = min(n, 64)
+    for m, extra in ((n, cfg), (k, {"per_tracer_launches": 1})):
+        ens = Ensemble(F.Harris(), m, max_rows=256, max_switch=16)
+        ens.configure(rtol=1e-8, atol=1e-8, gctimestep=0.5, **extra)
+        ens.set_particles(w["pos"][:m], w["vel"][:m], 0.0, w["mass"][:m], w["charge"][:m])
+        ens.upload()
+        ens.adaptive_init()
+        ens.advance("adaptive", d[:m])
+        h = ens.download()
+        rows, mode, nrows, swt, swm = ens.rows()
+        nsw = np.minimum(h["nswitch"][:k], 16)
+        out.append([h[a][..., :k].copy() for a in ("s", "t_row", "tcur", "mu", "status", "mode", "naccept", "nfcn", "nswitch")] +
+                   [nrows[:k].copy()] + [rows[i, :nrows[i]].copy() for i in range(k)] +
+                   [mode[i, :nrows[i]].copy() for i in range(k)] + [swt[i, :nsw[i]].copy() for i in range(k)])
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
