@@ -731,8 +731,14 @@ static int advance_impl(Ctx* c, int kind, const double* delta, double delta_all,
   const bool dense = c->cfg.dense_output != 0;
   if (dense && kind != RAPT_KIND_PARTICLE && c->max_rows < 18)
     return fail(c, RAPT_ERR_INVALID, "dense output needs max_rows >= 18 (a step may cover 17 output times)");
+  // k_gc32 takes one block an SM, as large as the ensemble fills (its warps keep in
+  // step, fp32_kernels.cuh), unless a block size is asked for; in Adaptive rounds the
+  // particle kernel has to find room on the same SMs, and blocks stay small.
+  int block_g = block;
+  if (f32 && kind == RAPT_KIND_GC && c->cfg.threads_per_block <= 0 && !c->cfg.per_tracer_launches)
+    block_g = (int)std::min<int64_t>(1024, 128 * ((c->n + 128 * c->num_sms - 1) / (128 * (int64_t)c->num_sms)));
   int bps_g = dense ? T.occ_gc_dense(block)
-                    : (tab != 0 ? T.occ_gc[tab](block) : (f32 ? T.occ_gc32_lrn[lrn](block) : T.occ_gc_lrn[lrn](block)));
+                    : (tab != 0 ? T.occ_gc[tab](block) : (f32 ? T.occ_gc32_lrn[lrn](block_g) : T.occ_gc_lrn[lrn](block)));
   if (c->cfg.blocks_per_sm > 0) {
     bps_p = std::min(bps_p, c->cfg.blocks_per_sm);
     bps_g = std::min(bps_g, c->cfg.blocks_per_sm);
@@ -748,7 +754,7 @@ static int advance_impl(Ctx* c, int kind, const double* delta, double delta_all,
   if (kind != RAPT_KIND_PARTICLE && c->cfg.gctimestep == 0) {
     // bounce-period cadence: one field-line scratch slot per thread of a grid
     const size_t threads =
-        c->cfg.per_tracer_launches ? 32 : (size_t)c->num_sms * (size_t)std::max(bps_g, bps_a) * block;
+        c->cfg.per_tracer_launches ? 32 : (size_t)c->num_sms * (size_t)std::max(bps_g * block_g, bps_a * block);
     const size_t bytes = threads * (size_t)P.fl_stride * sizeof(double);
     if (c->fl_bytes < bytes) {
       cudaFree(c->fl_scratch);
@@ -767,16 +773,16 @@ static int advance_impl(Ctx* c, int kind, const double* delta, double delta_all,
   // other lanes working in teams (the FP64 kernels; team_lanes in launch.h).
   P.lanes_p = 32;
   P.lanes_g = f32 || tab != 0 ? 32 : team_lanes(c->n, c->num_sms, c->field.model);
-  auto grid_of = [&](int bps, int lanes) {
-    const int64_t warps = (c->n + lanes - 1) / lanes, blocks = (warps * 32 + block - 1) / block;
+  auto grid_of = [&](int bps, int lanes, int threads) {
+    const int64_t warps = (c->n + lanes - 1) / lanes, blocks = (warps * 32 + threads - 1) / threads;
     return (int)std::min<int64_t>((int64_t)c->num_sms * bps, blocks);
   };
   const bool hand = bps_a >= 2;
   // otherwise an Adaptive round's two kernels run side by side: each takes half of the SMs' blocks
   const bool both = kind == RAPT_KIND_ADAPTIVE && !hand;
-  const int grid_a = 2 * std::max(grid_of(bps_a / 2, P.lanes_p), grid_of(bps_a / 2, P.lanes_g));
-  const int grid_p = grid_of(both ? (bps_p + 1) / 2 : bps_p, P.lanes_p);
-  const int grid_g = grid_of(both ? (bps_g + 1) / 2 : bps_g, P.lanes_g);
+  const int grid_a = 2 * std::max(grid_of(bps_a / 2, P.lanes_p, block), grid_of(bps_a / 2, P.lanes_g, block));
+  const int grid_p = grid_of(both ? (bps_p + 1) / 2 : bps_p, P.lanes_p, block);
+  const int grid_g = grid_of(both ? (bps_g + 1) / 2 : bps_g, P.lanes_g, block_g);
 
   CK(cudaEventRecord(c->ev0, s));
   if (resume) k_clear_rows_full<<<(unsigned)((N + 255) / 256), 256, 0, s>>>(E);
@@ -832,6 +838,7 @@ static int advance_impl(Ctx* c, int kind, const double* delta, double delta_all,
     }
     if (kind != RAPT_KIND_PARTICLE) {
       a.grid = gg;
+      a.block = blk == 32 ? 32 : block_g;
       a.stream = s;
       CK(dense ? T.gc_dense(a) : (tab != 0 ? T.gc[tab](a) : (f32 ? T.gc32_lrn[lrn](a) : T.gc_lrn[lrn](a))));
       ++kl;

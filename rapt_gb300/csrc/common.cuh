@@ -123,6 +123,25 @@ struct Scratch {
   unsigned long long accepted, rejected, rhs, switches, done, failed;
 };
 
+// (double)x, exactly, in integer instructions: a conversion instruction issues on
+// the FP64 pipe, 64 cycles a warp. Zeros, subnormals, infinities and NaN take it.
+__device__ __forceinline__ double widen(float x) {
+  const unsigned u = __float_as_uint(x), e = u & 0x7f800000u;
+  if (e == 0u || e == 0x7f800000u) return (double)x;
+  return __hiloint2double((int)((u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + 0x38000000u)), (int)(u << 29));
+}
+// max(a, b) of numbers that are not negative, compared as integers (a NaN is larger).
+__device__ __forceinline__ double max_nonneg(double a, double b) {
+  return __double_as_longlong(a) < __double_as_longlong(b) ? b : a;
+}
+// 0.1 |h| <= |t| u, Hairer's test for a vanished step (u about 2^-52): decided by
+// the exponents unless h is within a few binades of it.
+__device__ __forceinline__ bool step_vanished(double h, double t, double u) {
+  const int eh = (__double2hiint(h) >> 20) & 0x7ff, et = (__double2hiint(t) >> 20) & 0x7ff;
+  if (eh > et - 44 && eh != 0x7ff && et != 0x7ff && eh != 0) return false;
+  return 0.1 * fabs(h) <= fabs(t) * u;
+}
+
 // FP64 reciprocal and square root for quantities that need about 14 digits
 // (error norms, tolerance scales): the FP32 approximation (one MUFU
 // instruction) refined by one Newton-Raphson step in FP64, which squares its
@@ -145,13 +164,13 @@ __device__ __forceinline__ float rsqrt_approx_f32(float x) {
 __device__ __forceinline__ double rcp_nr(double x) {
   const float xf = (float)x;
   if (!(fabsf(xf) > 1e-36f && fabsf(xf) < 1e36f)) return 1.0 / x;
-  const double y = (double)rcp_approx_f32(xf);
+  const double y = widen(rcp_approx_f32(xf));
   return fma(y, fma(-x, y, 1.0), y);  // y (2 - x y)
 }
 __device__ __forceinline__ double sqrt_nr(double x) {
   const float xf = (float)x;
   if (!(xf > 1e-36f && xf < 1e36f)) return sqrt(x);
-  const double y = (double)rsqrt_approx_f32(xf);
+  const double y = widen(rsqrt_approx_f32(xf));
   const double s = x * y;                   // sqrt(x) to 2^-23
   return fma(0.5 * y, fma(-s, s, x), s);    // s + (x - s^2) / (2 sqrt(x))
 }

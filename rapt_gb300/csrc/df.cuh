@@ -19,7 +19,7 @@ struct DF {
 __device__ __forceinline__ DF df(float a) { return DF{a, 0.f}; }
 __device__ __forceinline__ DF df_from_double(double v) {
   const float h = (float)v;
-  return DF{h, (float)(v - (double)h)};
+  return DF{h, (float)(v - widen(h))};
 }
 __device__ __forceinline__ double df_to_double(DF a) { return (double)a.hi + (double)a.lo; }
 __device__ __forceinline__ float df_f(DF a) { return a.hi + a.lo; }

@@ -434,7 +434,7 @@ struct GcRHSdf {
 __device__ __forceinline__ double err_ratio(double e_si, DF y0, DF y1, double scale, double rtol, double atol,
                                            double floor = 0.0) {
   const float ym = fmaxf(fabsf(y0.hi), fabsf(y1.hi));
-  return e_si * rcp_nr(fmax(fma(rtol * scale, (double)ym, atol), floor));
+  return e_si * rcp_nr(max_nonneg(fma(rtol * scale, widen(ym), atol), floor));
 }
 
 // The DOPRI5 tableau as float-float pairs in constant memory (rows as kDp5A).
@@ -455,10 +455,10 @@ static __constant__ DFpair kDp5Adf[7][6] = {
 // the right-hand side (float-float field, stencil and equations) is emitted
 // once instead of six times, which keeps the kernel inside the instruction
 // cache at the high occupancy this form runs at.
-template <int NV, class F>
+template <int NV, class F, class Sync>
 __device__ __forceinline__ void dopri5_attempt_df_rolled(const F& f, double x, const DF* y, const DF* k1, double h,
-                                                         const double* scale, double rtol, double atol, DF* y1,
-                                                         DF* k7, double& err) {
+                                                         double last_scale, double rtol, double atol, DF* y1,
+                                                         DF* k7, double& err, const Sync& sync) {
   using namespace dp5;
   const DF hd = dfd(h);
   DF k2[NV], k3[NV], k4[NV], k5[NV], k6[NV], yt[NV], kt[NV];
@@ -466,6 +466,7 @@ __device__ __forceinline__ void dopri5_attempt_df_rolled(const F& f, double x, c
   for (int i = 0; i < NV; ++i) k2[i] = k3[i] = k4[i] = k5[i] = k6[i] = DF{0.f, 0.f};
 #pragma unroll 1
   for (int s = 1; s <= 6; ++s) {
+    sync();
     const DFpair* A = kDp5Adf[s];
     DF acc[NV];
     // only the slopes of row s (k1..k_s; the last row skips k2): warp-uniform
@@ -532,7 +533,7 @@ __device__ __forceinline__ void dopri5_attempt_df_rolled(const F& f, double x, c
     const float d = (y1[i].hi - y[i].hi) + (y1[i].lo - y[i].lo);
     dp2 = fmaf(d, d, dp2);
   }
-  const double pfloor = 3e-9 * (double)sqrtf(dp2);
+  const double pfloor = 3e-9 * widen(sqrtf(dp2));
   double e = 0.0;
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
@@ -542,7 +543,8 @@ __device__ __forceinline__ void dopri5_attempt_df_rolled(const F& f, double x, c
     ei = fmaf((float)e5, dk(k5[i]), ei);
     ei = fmaf((float)e6, dk(k6[i]), ei);
     ei = fmaf((float)e7, dk(k7[i]), ei);
-    const double r = err_ratio((double)ei * (h * scale[i]), y[i], y1[i], scale[i], rtol, atol, i < 3 ? pfloor : 0.0);
+    const double scale = i < NV - 1 ? 1.0 : last_scale;  // positions are in metres
+    const double r = err_ratio(widen(ei) * (h * scale), y[i], y1[i], scale, rtol, atol, i < 3 ? pfloor : 0.0);
     e = fma(r, r, e);
   }
   err = sqrt_nr(e * (1.0 / NV));
@@ -671,7 +673,8 @@ struct StepFactorF32 {
   __device__ __forceinline__ void reset(float beta) { inv_facold_beta = exp2f(-beta * __log2f(1e-4f)); }
   // err of an attempt -> the factor h_new / h after acceptance
   __device__ __forceinline__ float accept_factor(double err, float expo1, float safe, float facc1, float facc2) {
-    fac11 = exp2f(expo1 * __log2f((float)fmax(err, 1e-30)));
+    const float e = (float)err;  // rounding is monotonic: the maxima may be taken after it
+    fac11 = exp2f(expo1 * __log2f(fmaxf(e, 1e-30f)));
     const float fac = fmaxf(facc2, fminf(facc1, fac11 * inv_facold_beta * __fdividef(1.f, safe)));
     return __fdividef(1.f, fac);
   }
@@ -680,7 +683,7 @@ struct StepFactorF32 {
     return __fdividef(1.f, fminf(facc1, fac11 * __fdividef(1.f, safe)));
   }
   __device__ __forceinline__ void accepted(double err, float beta) {
-    inv_facold_beta = exp2f(-beta * __log2f((float)fmax(err, 1e-4)));
+    inv_facold_beta = exp2f(-beta * __log2f(fmaxf((float)err, 1e-4f)));
   }
 };
 

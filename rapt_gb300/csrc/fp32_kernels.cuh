@@ -243,14 +243,48 @@ __global__ void __launch_bounds__(128, 2) k_particle32(DevEnsemble E, const __gr
   st.flush(S);
 }
 
+// The warps of a block that share a sub-partition (warp index mod 4) and meet at a
+// barrier at every stage. Off (the warps go on by themselves) in blocks where a
+// sub-partition has only a few warps of the block.
+struct StageGroup {
+  bool on;
+  // whether any warp of the group has a tracer left: they stay together until none has
+  __device__ __forceinline__ bool any(bool busy) const {
+    if (!on) return busy;
+    unsigned r;
+    asm volatile(
+        "{\n .reg .pred p, q;\n setp.ne.u32 p, %1, 0;\n barrier.cta.red.or.pred q, %2, %3, p;\n"
+        " selp.u32 %0, 1, 0, q;\n}"
+        : "=r"(r)
+        : "r"((unsigned)busy), "r"(((threadIdx.x >> 5) & 3u) + 1u), "r"(blockDim.x >> 2)
+        : "memory");
+    return r != 0u;
+  }
+  __device__ __forceinline__ void operator()() const {
+    if (!on) return;
+    __syncwarp();
+    asm volatile("barrier.cta.sync %0, %1;" ::"r"(((threadIdx.x >> 5) & 3u) + 1u), "r"(blockDim.x >> 2) : "memory");
+  }
+};
+
 template <int M, int LRN = 0>
 // LRN: 0 plain controller, 1 training-sample collection, 2 MLP step proposals.
-// 8 blocks of 128 threads per SM, 64 registers: the balance between resident
-// warps (the float-float stages are long dependent FP32 chains) and the
-// local-memory traffic of spills. Measured on the 1M guiding-centre step
-// (FP32 / learned + FP32 accepted steps/s): 4 blocks/SM 1.44e9 / 1.04e9,
-// 6: 1.45e9 / 1.15e9, 8: 1.51e9 / 1.21e9, 12: 1.30e9 / 1.04e9, 16: 0.95e9 / 0.79e9.
-__global__ void __launch_bounds__(128, 8) k_gc32(DevEnsemble E, const __grid_constant__ KParams P, Scratch* S) {
+// 64 registers, 32 warps an SM: the balance between resident warps (the float-float
+// stages are long dependent FP32 chains) and the local-memory traffic of spills
+// (16 warps: 0.85 of the rate, 64: 0.64).
+// What bounds it: instruction fetch. A stage is some 30 KB of straight-line code, and
+// warps that are each somewhere else in it stall on the instruction cache first
+// (stall no_instruction 5.8 a issue, FP32 pipe 40 %, FP64 pipe 36 %). So the warps of
+// a block that share a sub-partition meet at a barrier at every stage and go through
+// the same code together: no_instruction 0.2, kernel 15.9 -> 14.4 ms (262,144 guiding
+// centres) and 153 -> 126 ms (learned, 1M). Measured on the same two: barriers once
+// an attempt 14.5 / 129; blocks of 512 (4 warps a group) 15.1 / 147, of 256
+// 15.9 / 154: the more warps share the fetches the better; two warps to a
+// sub-partition (blocks of 256) gain nothing and go on by themselves. The warps' first
+// tracers are dealt out over the blocks: taken by arrival, one block had the longest
+// 1,024 of an ensemble that fills the GPU once (150,000 guiding centres 18.9 -> 20.0 ms
+// by arrival, 17.9 dealt out).
+__global__ void __launch_bounds__(1024, 1) k_gc32(DevEnsemble E, const __grid_constant__ KParams P, Scratch* S) {
   int64_t idx = -1;
   bool exhausted = false;
   long long budget = P.budget;
@@ -271,6 +305,7 @@ __global__ void __launch_bounds__(128, 8) k_gc32(DevEnsemble E, const __grid_con
   StepFactorF32 ctl{1.f, 1.f};
   bool reject = false, last = false;
   int nst = 0, nacc_int = 0;
+  bool dealt = false;
 
   constexpr float beta = 0.04f, safe = 0.9f;
   constexpr float expo1 = 0.2f - beta * 0.75f, facc1 = 1.0f / 0.2f, facc2 = 1.0f / 10.0f;
@@ -334,15 +369,16 @@ __global__ void __launch_bounds__(128, 8) k_gc32(DevEnsemble E, const __grid_con
   };
 
   for (;;) {
-    warp_refill(&S->queue[1], E, RAPT_MODE_GC, 32, idx, exhausted, load);
-    if (__all_sync(kFull, idx < 0)) break;
+    warp_refill(&S->queue[1], E, RAPT_MODE_GC, 32, idx, exhausted, load, &dealt);
+    const bool busy = !__all_sync(kFull, idx < 0);
+    const StageGroup group{blockDim.x >= 512 && blockDim.x % 128 == 0};
+    if (!group.any(busy)) break;
     lr.infer(P, h);
-    if (idx < 0) continue;
 
     const GcRHSdf<M> rhs{P.f, kmu, mcq, muq, qmc, P.enforce_eq != 0};
-    bool release = false;
-
-    if (!in_interval) {
+    bool start = false;
+    if (idx >= 0 && !in_interval) {
+      start = true;
       if (!(seg_ok && rt < stop)) {
         bool more = false;
         if (P.kind == RAPT_KIND_ADAPTIVE && status != RAPT_ST_NONFINITE && status != RAPT_ST_BAD_INPUT &&
@@ -361,11 +397,18 @@ __global__ void __launch_bounds__(128, 8) k_gc32(DevEnsemble E, const __grid_con
           if (status != RAPT_ST_OK) st.fail++;
           store(idx, false);
           idx = -1;
-          continue;
+          start = false;
         }
       }
-      if (budget <= 0) { store(idx, true); idx = -1; exhausted = true; st.pend++; continue; }
-      if (nrows + 2 > P.max_rows) { status = RAPT_ST_ROWS_FULL; store(idx, true); idx = -1; continue; }
+      if (start && budget <= 0) { store(idx, true); idx = -1; exhausted = true; st.pend++; start = false; }
+      if (start && nrows + 2 > P.max_rows) {
+        status = RAPT_ST_ROWS_FULL;
+        store(idx, true);
+        idx = -1;
+        start = false;
+      }
+    }
+    if (start) {
       xend = rt + dt;
       hmax = fabs(xend - rt);
       posneg = copysign(1.0, xend - rt);
@@ -393,21 +436,32 @@ __global__ void __launch_bounds__(128, 8) k_gc32(DevEnsemble E, const __grid_con
       in_interval = true;
     }
 
-    bool ended = false;
+    bool ended = false, attempt = false;
     int fail = 0;
-    if (nst > P.nsteps) { ended = true; fail = RAPT_ST_MAXSTEPS; }
-    else if (0.1 * fabs(h) <= fabs(rt) * kUround) { ended = true; fail = RAPT_ST_HMIN; }
-    else {
+    if (idx >= 0) {
+      if (nst > P.nsteps) { ended = true; fail = RAPT_ST_MAXSTEPS; }
+      else if (step_vanished(h, rt, kUround)) { ended = true; fail = RAPT_ST_HMIN; }
+      else attempt = true;
+    }
+    if (attempt) {
       if ((rt + 1.01 * h - xend) * posneg > 0.0) { lr.before_clip(h); h = xend - rt; last = true; }
       ++nst;
       --budget;
-      DF y1[4], k7[4];
-      double err;
-      dopri5_attempt_df_rolled<4>(rhs, rt, y, k1, h, scale, P.rtol, P.atol, y1, k7, err);
+    }
+    DF y1[4], k7[4];
+    double err = 0.0;
+    // all lanes of a warp with an attempt to make go through it; the group's other
+    // warps meet it at the stages
+    if (__any_sync(kFull, attempt)) {
+      dopri5_attempt_df_rolled<4>(rhs, rt, y, k1, h, scale[3], P.rtol, P.atol, y1, k7, err, group);
+    } else {
+      for (int s = 0; s < 6; ++s) group();
+    }
+    if (attempt) {
       nfcn += 6;
       st.rhs += 6;
       lr.on_attempt(P, h, err, last);
-      double hnew = h * (double)ctl.accept_factor(err, expo1, safe, facc1, facc2);
+      double hnew = h * widen(ctl.accept_factor(err, expo1, safe, facc1, facc2));
       if (left_grid<M>(err)) {
         ended = true;
         fail = RAPT_ST_OUT_OF_GRID;
@@ -425,7 +479,7 @@ __global__ void __launch_bounds__(128, 8) k_gc32(DevEnsemble E, const __grid_con
           h = hnew;
           ended = true;
         } else {
-          if (fabs(hnew) > hmax) hnew = posneg * hmax;
+          if (__double_as_longlong(fabs(hnew)) > __double_as_longlong(hmax)) hnew = posneg * hmax;
           if (reject) hnew = posneg * fmin(fabs(hnew), fabs(h));
           reject = false;
           h = hnew;
@@ -435,7 +489,7 @@ __global__ void __launch_bounds__(128, 8) k_gc32(DevEnsemble E, const __grid_con
                      y[0].hi, y[1].hi, y[2].hi,
                      y[3].hi, vs, interval_progress(xend, rt, hmax));
       } else {
-        hnew = h * (double)ctl.reject_factor(safe, facc1);
+        hnew = h * widen(ctl.reject_factor(safe, facc1));
         reject = true;
         if (nacc_int >= 1) { ++nrej; st.rej++; }
         last = false;
@@ -483,16 +537,13 @@ __global__ void __launch_bounds__(128, 8) k_gc32(DevEnsemble E, const __grid_con
           E.status[idx] = status; E.flags[idx] = flags; E.nrows[idx] = nrows; E.nswitch[idx] = nswitch;
           E.nseg[idx] = nseg; E.seg_active[idx] = 0;
           idx = -1;
-          continue;
+        } else {
+          flags |= RAPT_FLAG_RAISED | RAPT_FLAG_DONE;
+          st.done++;
+          store(idx, false);
+          idx = -1;
         }
-        flags |= RAPT_FLAG_RAISED | RAPT_FLAG_DONE;
-        st.done++;
-        release = true;
       }
-    }
-    if (release) {
-      store(idx, false);
-      idx = -1;
     }
   }
   st.flush(S);

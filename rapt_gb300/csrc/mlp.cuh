@@ -347,7 +347,7 @@ struct StepLearner {
         if (rej_before) cap = fminf(cap, __fdividef(fh, fhn));
         hctl = hnew;
         rcap = cap;
-        hnew *= (double)fminf(rlast, cap);
+        hnew *= widen(fminf(rlast, cap));
       }
     }
     if (!coll && !coll_sw && !inf) return;
@@ -440,7 +440,7 @@ struct StepLearner {
         mlp_forward_staged(P.mlp_w, P.mlp_p, sm, o);
         if (want) {
           rlast = __expf(fminf(fmaxf(o[0], -3.f), 3.f)) * P.learn_scale;
-          if (pend_apply) h = hctl * (double)fminf(rlast, rcap);
+          if (pend_apply) h = hctl * widen(fminf(rlast, rcap));
         }
         want = false;
       }

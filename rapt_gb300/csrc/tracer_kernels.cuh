@@ -229,9 +229,12 @@ struct LaneStats {
 // of a launch hold the shortest tracers). Must be called by all 32 lanes.
 // lanes > 0: only the first `lanes` lanes take tracers (small ensembles spread
 // over more warps, whose other lanes work in teams).
+// dealt: for grids that deal the warps' first tracers out by warp and block index
+// instead of by arrival (false until that is done; the queue's head counts from the
+// positions dealt); null: by arrival.
 template <class LoadFn>
 __device__ __forceinline__ void warp_refill(unsigned long long* queue, const DevEnsemble& E, int mode, int lanes,
-                                            int64_t& idx, bool& exhausted, LoadFn&& load) {
+                                            int64_t& idx, bool& exhausted, LoadFn&& load, bool* dealt = nullptr) {
   const int lane = threadIdx.x & 31;
   const bool takes = lanes <= 0 || lane < lanes;
   for (;;) {
@@ -240,8 +243,13 @@ __device__ __forceinline__ void warp_refill(unsigned long long* queue, const Dev
     if (m == 0u) break;
     const int leader = __ffs(m) - 1;
     unsigned long long base = 0ull;
-    if (lane == leader) base = atomicAdd(queue, (unsigned long long)__popc(m));
-    base = __shfl_sync(kFull, base, leader);
+    if (dealt && !*dealt) {
+      base = ((unsigned long long)(threadIdx.x >> 5) * gridDim.x + blockIdx.x) * 32ull;
+      *dealt = true;
+    } else {
+      if (lane == leader) base = atomicAdd(queue, (unsigned long long)__popc(m));
+      base = __shfl_sync(kFull, base, leader) + (dealt ? (unsigned long long)gridDim.x * blockDim.x : 0ull);
+    }
     if (need) {
       const unsigned long long q = base + (unsigned long long)__popc(m & ((1u << lane) - 1u));
       if (q >= (unsigned long long)E.n) {
