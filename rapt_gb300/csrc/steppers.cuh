@@ -74,7 +74,9 @@ constexpr double a21 = 5.26001519587677318785587544488e-2, a31 = 1.9725056984537
 // Automatic initial step size (Hairer's HINIT): an explicit Euler step probes
 // the second derivative; h0 such that h^iord * max(|f|, |f'|) = 0.01.
 // f0 = f(x, y) is supplied (FSAL); one RHS evaluation.
-template <int NV, class F>
+// ORD8 (DOP853's 1/8): the eighth root of the larger of two roots, taken as one
+// sixteenth root.
+template <int NV, bool ORD8 = false, class F>
 __device__ __forceinline__ double hinit(const F& f, double x, const double* y, const double* f0, double posneg,
                                         double iord_inv, double hmax, double rtol, double atol) {
   double dnf = 0.0, dny = 0.0, isk[NV];
@@ -97,6 +99,14 @@ __device__ __forceinline__ double hinit(const F& f, double x, const double* y, c
   for (int i = 0; i < NV; ++i) {
     const double a = (f1[i] - f0[i]) * isk[i];
     der2 += a * a;
+  }
+  if (ORD8) {
+    const double ih = 1.0 / h, q = fmax(der2 * ih * ih, dnf);
+    if (q > 1e-30 && q < 1e300) {
+      const double h1 = rsixteenth_root(q * 1e4);
+      h = fmin(fmin(100.0 * fabs(h), h1), hmax);
+      return copysign(h, posneg);
+    }
   }
   der2 = sqrt(der2) / h;
   const double der12 = fmax(fabs(der2), sqrt(dnf));
@@ -292,7 +302,7 @@ __device__ __forceinline__ void dop853_attempt(const F& f, double x, const doubl
     const double bs = b1 * k1[i] + b6 * k6[i] + b7 * k7[i] + b8 * k8[i] + b9 * k9[i] + b10 * k10[i] +
                       b11 * k2[i] + b12 * k3[i];
     y1[i] = y[i] + h * bs;
-    const double isk = 1.0 / (atol + rtol * fmax(fabs(y[i]), fabs(y1[i])));
+    const double isk = 1.0 / (atol + rtol * max_nonneg(fabs(y[i]), fabs(y1[i])));
     const double r3 = (bs - bhh1 * k1[i] - bhh2 * k9[i] - bhh3 * k3[i]) * isk;
     const double r5 = (er1 * k1[i] + er6 * k6[i] + er7 * k7[i] + er8 * k8[i] + er9 * k9[i] + er10 * k10[i] +
                        er11 * k2[i] + er12 * k3[i]) * isk;

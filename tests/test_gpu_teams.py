@@ -103,3 +103,23 @@ def test_adaptive_hand_over(n, cfg):
                    [mode[i, :nrows[i]].copy() for i in range(k)] + [swt[i, :nsw[i]].copy() for i in range(k)])
     for a, b in zip(*out):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("n", [1, 33, 609, 5000])
+@pytest.mark.parametrize("tableau", [0, 1])
+def test_particles_spread(n, tableau):
+    """Few particles a warp (small ensembles) against full warps."""
+    from rapt_gb300 import Ensemble
+    w = W.config1(BIG)
+    out = []
+    for m in (n, BIG):
+        ens = Ensemble(F.EarthDipole(), m, max_rows=32)
+        ens.configure(rtol=1e-8, atol=1e-8, cyclotronresolution=10, tableau=tableau)
+        ens.set_particles(w["pos"][:m], w["vel"][:m], 0.0, w["mass"][:m], w["charge"][:m])
+        ens.upload()
+        ens.advance("particle", 0.02)
+        h = ens.download()
+        k = min(n, 128)
+        out.append([h[a][..., :k].copy() for a in ("s", "t_row", "status", "naccept", "nreject", "nfcn")])
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
