@@ -62,6 +62,8 @@ struct Ctx {
   int64_t mlp_t = 0;  // Adam step count
   double* fl_scratch = nullptr;  // field-line traces of the bounce-period cadence
   size_t fl_bytes = 0;
+  char* share = nullptr;         // k_gc_share: state of given tracers, mailboxes, waiting ring
+  size_t share_bytes = 0;
   float* samp = nullptr;
   unsigned long long* samp_count = nullptr;
   int64_t samp_cap = 0;
@@ -224,10 +226,11 @@ __global__ void k_prepare(DevEnsemble E, const double* delta, double delta_all, 
   E.t_int[k] = E.t_row[k];
 }
 
-// Start of a k_adaptive launch: the tracers still to be advanced, counted.
-__global__ void k_count_left(DevEnsemble E, Scratch* S) {
+// Start of a k_adaptive or k_gc_share launch: the tracers still to be advanced, counted.
+__global__ void k_count_left(DevEnsemble E, Scratch* S, bool gc_only) {
   const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const bool left = k < E.n && !(E.flags[k] & RAPT_FLAG_DONE) && E.status[k] != RAPT_ST_ROWS_FULL;
+  const bool left = k < E.n && !(E.flags[k] & RAPT_FLAG_DONE) && E.status[k] != RAPT_ST_ROWS_FULL &&
+                    (!gc_only || E.mode[k] == RAPT_MODE_GC);
   const unsigned long long c = (unsigned long long)__syncthreads_count(left);
   if (threadIdx.x == 0 && c) {
     atomicAdd(&S->pending, c);
@@ -323,6 +326,7 @@ void rapt_ctx_destroy(void* ctx) {
   cudaFree(c->tmp);
   cudaFree(c->mlp_block);
   cudaFree(c->fl_scratch);
+  cudaFree(c->share);
   cudaFree(c->samp_count);  // base of the sample allocation
   cudaFree(c->grid);
   cudaFreeHost(c->h_pending);
@@ -804,6 +808,36 @@ static int advance_impl(Ctx* c, int kind, const double* delta, double delta_all,
   const int grid_p = grid_of(both ? (bps_p + 1) / 2 : bps_p, P.lanes_p, block);
   const int grid_g = grid_of(both ? (bps_g + 1) / 2 : bps_g, P.lanes_g, block_g);
 
+  // Guiding centres in the plain form, from one warp a sub-partition up to 32: tracers
+  // shared between the warps at the end of the launch (k_gc_share). One block an SM at
+  // least, so that every sub-partition has a warp that takes (two: 10,000 tracers 10.4 ->
+  // 12.5 ms, they share the FP64 pipe). Above 32 warps a sub-partition the end of the
+  // launch is 1 % of it. Not with a step budget, whose lanes stop between intervals, and
+  // without memory for it the plain kernel runs.
+  int grid_s = 0;
+  size_t share_head = 0;  // bytes of the mailboxes and the ring
+  if (kind == RAPT_KIND_GC && form == RAPT_FORM_PLAIN && tab == 0 && lrn == 0 && !dense && !c->cfg.per_tracer_launches &&
+      c->cfg.max_steps_per_launch <= 0 && P.lanes_g == 32 && c->n <= 32ll * 32 * c->num_sms) {
+    int bps_s = T.occ_gc_share(block);
+    if (c->cfg.blocks_per_sm > 0) bps_s = std::min(bps_s, c->cfg.blocks_per_sm);
+    grid_s = std::max(grid_of(bps_s, 32, block), std::min(bps_s, 1) * c->num_sms);
+    const size_t warps = (size_t)grid_s * (block / 32);
+    share_head = (warps * (kMailWords + 1) * 4 + 255) / 256 * 256;
+    const size_t bytes = share_head + N * kMidWords * 8;
+    if (grid_s > 0 && c->share_bytes < bytes) {
+      cudaFree(c->share);
+      c->share = nullptr;
+      c->share_bytes = 0;
+      if (cudaMalloc(&c->share, bytes) == cudaSuccess) c->share_bytes = bytes;
+      else { cudaGetLastError(); grid_s = 0; }
+    }
+    if (grid_s > 0) {
+      E.mail = (int32_t*)c->share;
+      E.waitq = E.mail + warps * kMailWords;
+      E.mid = (double*)(c->share + share_head);
+    }
+  }
+
   CK(cudaEventRecord(c->ev0, s));
   if (resume) k_clear_rows_full<<<(unsigned)((N + 255) / 256), 256, 0, s>>>(E);
   else k_prepare<<<(unsigned)((N + 255) / 256), 256, 0, s>>>(E, d_delta, delta_all, kind);
@@ -839,10 +873,19 @@ static int advance_impl(Ctx* c, int kind, const double* delta, double delta_all,
       a.E.mode0 = Ev.mode;
     if (hand) {
       for (int i = 0; i < 2; ++i) CK(cudaMemsetAsync(Ev.ring[i], 0, (size_t)Ev.n * 4, s));
-      k_count_left<<<(unsigned)((Ev.n + 255) / 256), 256, 0, s>>>(Ev, c->scratch);
+      k_count_left<<<(unsigned)((Ev.n + 255) / 256), 256, 0, s>>>(Ev, c->scratch, false);
       CK(cudaGetLastError());
       a.grid = grid_a;
       CK(T.adaptive(a));
+      kl += 2;
+      return RAPT_OK;
+    }
+    if (grid_s > 0) {
+      CK(cudaMemsetAsync(Ev.mail, 0, share_head, s));
+      k_count_left<<<(unsigned)((Ev.n + 255) / 256), 256, 0, s>>>(Ev, c->scratch, true);
+      CK(cudaGetLastError());
+      a.grid = grid_s;
+      CK(T.gc_share(a));
       kl += 2;
       return RAPT_OK;
     }

@@ -109,8 +109,15 @@ struct DevEnsemble {
   // hand-over rings of k_adaptive, n entries each ([mode]: tracers that switched to
   // that mode, index + 1; 0: empty)
   int32_t* ring[2];
+  // sharing of tracers between the warps of a k_gc_share launch: state of tracers given
+  // away inside an interval (kMidWords arrays of n), a mailbox of kMailWords a warp, and
+  // the ring of the warps that wait (one entry a warp)
+  double* mid;
+  int32_t* mail;
+  int32_t* waitq;
 };
-constexpr int kRoundWords = 8;  // words of Scratch that are reset for every round
+constexpr int kMidWords = 9, kMailWords = 8;
+constexpr int kRoundWords = 10;  // words of Scratch that are reset for every round
 
 // Scratch words used by the persistent kernels (one block of device memory).
 struct Scratch {
@@ -120,6 +127,7 @@ struct Scratch {
   // read and write positions ([mode])
   unsigned long long remaining;
   unsigned long long ring_head[2], ring_tail[2];
+  unsigned long long wait_head, wait_tail;  // k_gc_share: positions in the ring of waiting warps
   unsigned long long accepted, rejected, rhs, switches, done, failed;
 };
 

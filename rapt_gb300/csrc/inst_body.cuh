@@ -35,6 +35,15 @@ int occ_gc(int block) {
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_gc<kM, TAB>, block, 0);
   return nb;
 }
+cudaError_t launch_gc_share(const LaunchArgs& a) {
+  k_gc_share<kM><<<a.grid, a.block, 0, a.stream>>>(a.E, a.P, a.S);
+  return cudaGetLastError();
+}
+int occ_gc_share(int block) {
+  int nb = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_gc_share<kM>, block, 0);
+  return nb;
+}
 cudaError_t launch_adaptive(const LaunchArgs& a) {
   k_adaptive<kM><<<a.grid, a.block, 0, a.stream>>>(a.E, a.P, a.S);
   return cudaGetLastError();
@@ -183,6 +192,8 @@ void RAPT_CAT(register_model_, RAPT_MODEL)(ModelTable* t) {
   t->rhs_eval = rhs_eval;
   t->adaptive_init = adaptive_init;
   t->bounce_period = bounce_period;
+  t->gc_share = launch_gc_share;
+  t->occ_gc_share = occ_gc_share;
   t->adaptive = launch_adaptive;
   t->occ_adaptive = occ_adaptive;
   t->gc_dense = launch_gc_dense;

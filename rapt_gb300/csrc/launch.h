@@ -66,6 +66,8 @@ struct ModelTable {
   RhsEvalFn rhs_eval;
   AdaptiveInitFn adaptive_init;
   BounceFn bounce_period;
+  LaunchFn gc_share;  // plain DOPRI5 form, tracers shared between warps
+  OccFn occ_gc_share;
   LaunchFn adaptive;  // both modes in one grid (plain FP64 form, DOP853 / DOPRI5)
   OccFn occ_adaptive;
   LaunchFn gc_dense;  // DOPRI5 guiding centres with dense output (rapt_config.dense_output)

@@ -275,19 +275,22 @@ __device__ __forceinline__ void hand_over(const DevEnsemble& E, Scratch* S, int 
   const unsigned long long at = atomicAdd(&S->ring_tail[mode], 1ull);
   atomicExch(&E.ring[mode][at % (unsigned long long)E.n], (int32_t)idx + 1);
 }
-__device__ __forceinline__ int64_t take_over(const DevEnsemble& E, Scratch* S, int mode) {
+__device__ __forceinline__ int64_t take_entry(int32_t* ring, unsigned long long entries, unsigned long long* head) {
   for (int tries = 0; tries < 4; ++tries) {
-    const unsigned long long at = *(volatile unsigned long long*)&S->ring_head[mode];
-    int32_t* e = &E.ring[mode][at % (unsigned long long)E.n];
+    const unsigned long long at = *(volatile unsigned long long*)head;
+    int32_t* e = &ring[at % entries];
     const int32_t v = *(volatile int32_t*)e;
     if (v == 0) return -1;
-    if (atomicCAS(&S->ring_head[mode], at, at + 1) == at) {
+    if (atomicCAS(head, at, at + 1) == at) {
       atomicExch(e, 0);
       __threadfence();
       return (int64_t)v - 1;
     }
   }
   return -1;
+}
+__device__ __forceinline__ int64_t take_over(const DevEnsemble& E, Scratch* S, int mode) {
+  return take_entry(E.ring[mode], (unsigned long long)E.n, &S->ring_head[mode]);
 }
 // A tracer has stopped for this launch; finished: it needs no further launch.
 __device__ __forceinline__ void retire(Scratch* S, bool finished) {
@@ -315,6 +318,87 @@ __device__ __forceinline__ void warp_take(const DevEnsemble& E, Scratch* S, int 
     if (lane == 0) left = *(volatile unsigned long long*)&S->remaining;
     if (__shfl_sync(kFull, left, 0) == 0ull) return;
     __nanosleep(1000);
+  }
+}
+
+// ---- sharing of tracers between the warps of a launch (k_gc_share)
+// A warp without a tracer enters the ring of waiting warps and polls its mailbox,
+// until a warp with many tracers gives it some, every tracer of the launch has stopped
+// or kPolls polls (1 us each at first, then 20) have passed; it then closes its mailbox.
+// Mailbox word 0: 0 open, -1 closed, -2 being filled, > 0 that many tracers in words 1..
+// All 32 lanes call these.
+template <class LoadFn>
+__device__ __forceinline__ void share_wait(const DevEnsemble& E, Scratch* S, int64_t& idx, LoadFn&& load) {
+  const int lane = threadIdx.x & 31;
+  const unsigned warps = gridDim.x * (blockDim.x >> 5), w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  int32_t* mail = E.mail + (size_t)w * kMailWords;
+  if (lane == 0) {
+    const unsigned long long at = atomicAdd(&S->wait_tail, 1ull);
+    atomicExch(&E.waitq[at % warps], (int32_t)w + 1);
+  }
+  for (int poll = 0; poll < kPolls + 4096; ++poll) {
+    int got = 0;
+    if (lane == 0) {
+      got = *(volatile int32_t*)mail;
+      if (got == 0 && (poll >= kPolls || *(volatile unsigned long long*)&S->remaining == 0ull))
+        got = atomicCAS(mail, 0, -1) == 0 ? -1 : 0;
+    }
+    got = __shfl_sync(kFull, got, 0);
+    if (got == -1) return;
+    if (got > 0) {
+      __threadfence();
+      __syncwarp();
+      if (lane < got) idx = *(volatile int32_t*)&mail[1 + lane];
+      __syncwarp();
+      if (lane == 0) atomicExch(mail, 0);
+      if (lane < got) load(idx);
+      __syncwarp();
+      return;
+    }
+    __nanosleep(poll < 4096 ? 1000 : 20000);
+  }
+}
+// A warp with more tracers than a round of TEAMS teams serves gives them to waiting
+// warps, TEAMS to each, where enough wait for it to get down to the MOST lanes that
+// work in teams: below that number each tracer less makes its right-hand sides
+// cheaper, above it a warp pays for 32 lanes whatever it holds.
+template <int TEAMS, int MOST, class StoreFn>
+__device__ __forceinline__ void share_give(const DevEnsemble& E, Scratch* S, int64_t& idx, bool in_interval,
+                                           StoreFn&& store_mid) {
+  const int lane = threadIdx.x & 31;
+  int held = __popc(__ballot_sync(kFull, idx >= 0));
+  if (held <= TEAMS) return;
+  long long waiting = 0;
+  if (lane == 0)
+    waiting = (long long)(*(volatile unsigned long long*)&S->wait_tail - *(volatile unsigned long long*)&S->wait_head);
+  waiting = __shfl_sync(kFull, waiting, 0);
+  if (waiting < (held > MOST ? (held - MOST + TEAMS - 1) / TEAMS : 1)) return;
+  const unsigned warps = gridDim.x * (blockDim.x >> 5);
+  unsigned can = __ballot_sync(kFull, idx >= 0 && in_interval);
+  while (held > TEAMS && can) {
+    int to = -1;
+    if (lane == 0) {
+      to = (int)take_entry(E.waitq, warps, &S->wait_head);
+      if (to >= 0 && atomicCAS(&E.mail[(size_t)to * kMailWords], 0, -2) != 0) to = -2;  // closed meanwhile
+    }
+    to = __shfl_sync(kFull, to, 0);
+    if (to == -1) break;
+    if (to == -2) continue;
+    const int g = min(min(TEAMS, held - TEAMS), __popc(can)), rank = __popc(can & ((1u << lane) - 1u));
+    int32_t* mail = E.mail + (size_t)to * kMailWords;
+    if ((can >> lane & 1u) && rank < g) {
+      store_mid(idx);
+      *(volatile int32_t*)&mail[1 + rank] = (int32_t)idx;
+      idx = -1;
+      __threadfence();
+    }
+    __syncwarp();
+    if (lane == 0) {
+      __threadfence();
+      atomicExch(mail, g);
+    }
+    for (int i = 0; i < g; ++i) can &= can - 1u;
+    held -= g;
   }
 }
 
@@ -618,9 +702,11 @@ __global__ void __launch_bounds__(128) k_particle(DevEnsemble E, const __grid_co
 // LRN (DOPRI5 only): 0 plain, 1 training-sample collection, 2 MLP step proposals
 // (a proposal replaces the controller's next step after an accepted step and
 // HINIT at the next interval; a rejected proposal falls back to the controller).
-template <int M, int TAB, int LRN, bool HAND>
+template <int M, int TAB, int LRN, bool HAND, bool SHARE>
 __device__ __forceinline__ void gc_body(const DevEnsemble& E, const KParams& P, Scratch* S) {
   static_assert(LRN == 0 || TAB == 0, "the step learner drives the DOPRI5 controller");
+  static_assert(!SHARE || (TAB == 0 && LRN == 0 && !HAND), "sharing: the plain DOPRI5 form");
+  constexpr bool COUNT = HAND || SHARE;  // tracers that stop are counted as they do
   int64_t idx = -1;
   bool exhausted = false, spent = false;
   long long budget = P.budget;
@@ -678,6 +764,19 @@ __device__ __forceinline__ void gc_body(const DevEnsemble& E, const KParams& P, 
     seg_ok = true;
     if (E.seg_active[k]) {
       stop = E.seg_stop[k]; dt = E.seg_dt[k];
+      if (SHARE && E.seg_active[k] == 2) {  // given away inside an interval
+        const double* m = E.mid + k;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) k1[i] = m[(size_t)i * E.n];
+        h = m[(size_t)4 * E.n]; facold = m[(size_t)5 * E.n]; xend = m[(size_t)6 * E.n]; hmax = m[(size_t)7 * E.n];
+        const long long c = __double_as_longlong(m[(size_t)8 * E.n]);
+        nst = (int)(c & 0x7fffffffll);
+        nacc_int = (int)(c >> 32 & 1);
+        reject = (c >> 33 & 1) != 0;
+        posneg = 1.0;
+        last = false;
+        k1_valid = in_interval = true;
+      }
     } else {
       begin_segment((P.kind == RAPT_KIND_ADAPTIVE && nseg > 0) ? delta - tcur : delta);
     }
@@ -695,9 +794,23 @@ __device__ __forceinline__ void gc_body(const DevEnsemble& E, const KParams& P, 
     E.seg_active[k] = active ? 1 : 0;
     E.seg_stop[k] = stop; E.seg_dt[k] = dt;
   };
+  // between two attempts of an interval (dt > 0, so posneg is 1, and last is not set)
+  auto store_mid = [&](int64_t k) {
+    store(k, true);
+    E.seg_active[k] = 2;
+    double* m = E.mid + k;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) m[(size_t)i * E.n] = k1[i];
+    m[(size_t)4 * E.n] = h; m[(size_t)5 * E.n] = facold; m[(size_t)6 * E.n] = xend; m[(size_t)7 * E.n] = hmax;
+    m[(size_t)8 * E.n] = __longlong_as_double((long long)nst | (long long)(nacc_int >= 1) << 32 | (long long)reject << 33);
+  };
 
   for (;;) {
     warp_refill(&S->queue[1], E, RAPT_MODE_GC, P.lanes_g, idx, exhausted, load);
+    if (SHARE) {
+      if (__all_sync(kFull, idx < 0)) share_wait(E, S, idx, load);
+      else share_give<GcTeam<M>::kTeams, GcTeam<M>::kMaxLanes>(E, S, idx, in_interval, store_mid);
+    }
     if (HAND) warp_take(E, S, RAPT_MODE_GC, P.lanes_g, idx, exhausted, spent, load);
     if (__all_sync(kFull, idx < 0)) break;
     lr.infer(P, h);
@@ -725,7 +838,7 @@ __device__ __forceinline__ void gc_body(const DevEnsemble& E, const KParams& P, 
           st.done++;
           if (status != RAPT_ST_OK) st.fail++;
           store(idx, false);
-          if (HAND) retire(S, true);
+          if (COUNT) retire(S, true);
           idx = -1;
           start = false;
         }
@@ -734,14 +847,14 @@ __device__ __forceinline__ void gc_body(const DevEnsemble& E, const KParams& P, 
         store(idx, true);
         idx = -1;
         exhausted = spent = true;
-        if (HAND) retire(S, false);
+        if (COUNT) retire(S, false);
         else st.pend++;
         start = false;
       }
       if (start && nrows + 2 > P.max_rows) {
         status = RAPT_ST_ROWS_FULL;
         store(idx, true);
-        if (HAND) retire(S, true);
+        if (COUNT) retire(S, true);
         idx = -1;
         start = false;
       }
@@ -915,7 +1028,7 @@ __device__ __forceinline__ void gc_body(const DevEnsemble& E, const KParams& P, 
           flags |= RAPT_FLAG_RAISED | RAPT_FLAG_DONE;
           st.done++;
           store(idx, false);
-          if (HAND) retire(S, true);
+          if (COUNT) retire(S, true);
           idx = -1;
         }
       }
@@ -926,7 +1039,21 @@ __device__ __forceinline__ void gc_body(const DevEnsemble& E, const KParams& P, 
 
 template <int M, int TAB, int LRN = 0>
 __global__ void __launch_bounds__(128) k_gc(DevEnsemble E, const __grid_constant__ KParams P, Scratch* S) {
-  gc_body<M, TAB, LRN, false>(E, P, S);
+  gc_body<M, TAB, LRN, false, false>(E, P, S);
+}
+
+// Guiding centres whose tracers move between the warps of the launch. A warp pays for a
+// right-hand side of 32 lanes as long as more lanes than GcTeam::kMaxLanes hold a
+// tracer, and its longest tracer keeps it there while other sub-partitions have run out
+// of work (grid of 16,384: SMs active for half of the launch, 31 of 90 ms of FP64
+// pipe). With teams, eight or more warps finish the same tracers several times sooner.
+// Nothing of a tracer's arithmetic depends on the warp it is in. Measured (kernel): 8,000 in the
+// double dipole 13.3 -> 10.0 ms, 16,384 13.4 -> 11.5, 32,768 22.3 -> 19.6, 65,536
+// 33.3 -> 33.0, 131,072 64.5 -> 63.9; 16,384 in a grid 90 -> 76 ms, at the bounce
+// cadence 15.5 -> 14.5.
+template <int M>
+__global__ void __launch_bounds__(128) k_gc_share(DevEnsemble E, const __grid_constant__ KParams P, Scratch* S) {
+  gc_body<M, 0, 0, false, true>(E, P, S);
 }
 
 // ---------------------------------------------------------------- Adaptive in one launch
@@ -941,7 +1068,7 @@ __global__ void __launch_bounds__(128) k_gc(DevEnsemble E, const __grid_constant
 template <int M>
 __global__ void __launch_bounds__(128) k_adaptive(DevEnsemble E, const __grid_constant__ KParams P, Scratch* S) {
   if (blockIdx.x < gridDim.x / 2) particle_body<M, 0, true>(E, P, S);
-  else gc_body<M, 0, 0, true>(E, P, S);
+  else gc_body<M, 0, 0, true, false>(E, P, S);
 }
 
 }  // namespace rapt

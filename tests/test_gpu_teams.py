@@ -123,3 +123,34 @@ def test_particles_spread(n, tableau):
         out.append([h[a][..., :k].copy() for a in ("s", "t_row", "status", "naccept", "nreject", "nfcn")])
     for a, b in zip(*out):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("n", [7297, 10007, 19457])
+@pytest.mark.parametrize("model", ["DoubleDipole", "CompressedDipole", "Harris", "Grid"])
+@pytest.mark.parametrize("cadence", [0.01, 0.07, 0.0])
+def test_shared_between_warps(model, n, cadence):
+    """Tracers given from warp to warp inside an interval against a launch in which
+    each stays where it began (a step budget, here far away, switches sharing off):
+    states, rows and counters, with several intervals and with one, and durations
+    that leave many warps without a tracer."""
+    if cadence == 0.0 and model not in ("DoubleDipole", "CompressedDipole"):
+        pytest.skip("a bounce needs mirror points")
+    from rapt_gb300 import Ensemble
+    w = W.config2(n, seed=9)
+    if model == "Harris":
+        w = dict(w, mass=np.full(n, W.m_pr), charge=np.full(n, W.e), v=np.linspace(3e5, 3e6, n), pos=W.config3(n, 2)["pos"])
+    delta = np.random.default_rng(4).choice([0.0, 0.01, 0.03, 0.06], n)
+    out = []
+    for budget in (0, 1 << 40):
+        ens = Ensemble(MODELS[model](), n, max_rows=64)
+        ens.configure(rtol=1e-7, atol=1e-7, gctimestep=cadence, bounceresolution=20.0, max_steps_per_launch=budget)
+        ens.set_guiding_centers(w["pos"], w["v"], pa=w["pa"], t0=0.5, mass=w["mass"], charge=w["charge"])
+        ens.upload()
+        st = ens.advance("gc", delta)
+        h = ens.download()
+        rows, _, nrows, _, _ = ens.rows()
+        out.append([h[a].copy() for a in ("s", "t_row", "tcur", "mu", "status", "flags", "naccept", "nreject", "nfcn")] +
+                   [nrows, np.where(np.arange(64)[None, :, None] < nrows[:, None, None], rows, 0.0),
+                    np.array([st[a] for a in ("accepted", "rejected", "rhs_evals", "done", "failed")])])
+    for a, b in zip(*out):
+        assert np.array_equal(a, b, equal_nan=a.dtype.kind == "f")
