@@ -809,17 +809,20 @@ static int advance_impl(Ctx* c, int kind, const double* delta, double delta_all,
   const int grid_g = grid_of(both ? (bps_g + 1) / 2 : bps_g, P.lanes_g, block_g);
 
   // Guiding centres in the plain form, from one warp a sub-partition up to 32: tracers
-  // shared between the warps at the end of the launch (k_gc_share). One block an SM at
-  // least, so that every sub-partition has a warp that takes (two: 10,000 tracers 10.4 ->
-  // 12.5 ms, they share the FP64 pipe). Above 32 warps a sub-partition the end of the
-  // launch is 1 % of it. Not with a step budget, whose lanes stop between intervals, and
-  // without memory for it the plain kernel runs.
+  // shared between the warps at the end of the launch (k_gc_share, k_gc_dense<M, true>).
+  // One block an SM at least, so that every sub-partition has a warp that takes (two:
+  // 10,000 tracers 10.4 -> 12.5 ms, they share the FP64 pipe). Above 32 warps a
+  // sub-partition the end of the launch is 1 % of it. Not in a grid with dense output (the
+  // compiler contracts a row's sums differently in the two kernels, by one unit in the last
+  // place, and a grid's steps follow it); not with a step budget, whose lanes stop between
+  // intervals; without memory for it the plain kernel runs.
   int grid_s = 0;
   size_t share_head = 0;  // bytes of the mailboxes and the ring
-  if (kind == RAPT_KIND_GC && form == RAPT_FORM_PLAIN && tab == 0 && lrn == 0 && !dense && !c->cfg.per_tracer_launches &&
-      c->cfg.max_steps_per_launch <= 0 && P.lanes_g == 32 && c->n <= 32ll * 32 * c->num_sms) {
-    int bps_s = T.occ_gc_share(block);
-    if (c->cfg.blocks_per_sm > 0) bps_s = std::min(bps_s, c->cfg.blocks_per_sm);
+  if (kind == RAPT_KIND_GC && form == RAPT_FORM_PLAIN && tab == 0 && lrn == 0 && !c->cfg.per_tracer_launches &&
+      c->cfg.max_steps_per_launch <= 0 && P.lanes_g == 32 && !(dense && c->field.model == RAPT_GRID) &&
+      c->n <= 32ll * 32 * c->num_sms) {
+    // (no more blocks than the plain kernel's, which the field-line scratch is sized for)
+    const int bps_s = std::min(dense ? T.occ_gc_dense_share(block) : T.occ_gc_share(block), bps_g);
     grid_s = std::max(grid_of(bps_s, 32, block), std::min(bps_s, 1) * c->num_sms);
     const size_t warps = (size_t)grid_s * (block / 32);
     share_head = (warps * (kMailWords + 1) * 4 + 255) / 256 * 256;
@@ -885,7 +888,7 @@ static int advance_impl(Ctx* c, int kind, const double* delta, double delta_all,
       k_count_left<<<(unsigned)((Ev.n + 255) / 256), 256, 0, s>>>(Ev, c->scratch, true);
       CK(cudaGetLastError());
       a.grid = grid_s;
-      CK(T.gc_share(a));
+      CK(dense ? T.gc_dense_share(a) : T.gc_share(a));
       kl += 2;
       return RAPT_OK;
     }

@@ -53,13 +53,15 @@ int occ_adaptive(int block) {
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_adaptive<kM>, block, 0);
   return nb;
 }
+template <bool SHARE>
 cudaError_t launch_gc_dense(const LaunchArgs& a) {
-  k_gc_dense<kM><<<a.grid, a.block, 0, a.stream>>>(a.E, a.P, a.S);
+  k_gc_dense<kM, SHARE><<<a.grid, a.block, 0, a.stream>>>(a.E, a.P, a.S);
   return cudaGetLastError();
 }
+template <bool SHARE>
 int occ_gc_dense(int block) {
   int nb = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_gc_dense<kM>, block, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_gc_dense<kM, SHARE>, block, 0);
   return nb;
 }
 cudaError_t launch_particle32(const LaunchArgs& a) {
@@ -196,8 +198,10 @@ void RAPT_CAT(register_model_, RAPT_MODEL)(ModelTable* t) {
   t->occ_gc_share = occ_gc_share;
   t->adaptive = launch_adaptive;
   t->occ_adaptive = occ_adaptive;
-  t->gc_dense = launch_gc_dense;
-  t->occ_gc_dense = occ_gc_dense;
+  t->gc_dense = launch_gc_dense<false>;
+  t->occ_gc_dense = occ_gc_dense<false>;
+  t->gc_dense_share = launch_gc_dense<true>;
+  t->occ_gc_dense_share = occ_gc_dense<true>;
   t->bc_start = bc_start;
   t->bc_interval = bc_interval;
   t->bc_eval = bc_eval;

@@ -127,8 +127,8 @@ def test_particles_spread(n, tableau):
 
 @pytest.mark.parametrize("n", [7297, 10007, 19457])
 @pytest.mark.parametrize("model", ["DoubleDipole", "CompressedDipole", "Harris", "Grid"])
-@pytest.mark.parametrize("cadence", [0.01, 0.07, 0.0])
-def test_shared_between_warps(model, n, cadence):
+@pytest.mark.parametrize("cadence,dense", [(0.01, 0), (0.07, 0), (0.0, 0), (0.01, 1), (0.0, 1)])
+def test_shared_between_warps(model, n, cadence, dense):
     """Tracers given from warp to warp inside an interval against a launch in which
     each stays where it began (a step budget, here far away, switches sharing off):
     states, rows and counters, with several intervals and with one, and durations
@@ -143,7 +143,8 @@ def test_shared_between_warps(model, n, cadence):
     out = []
     for budget in (0, 1 << 40):
         ens = Ensemble(MODELS[model](), n, max_rows=64)
-        ens.configure(rtol=1e-7, atol=1e-7, gctimestep=cadence, bounceresolution=20.0, max_steps_per_launch=budget)
+        ens.configure(rtol=1e-7, atol=1e-7, gctimestep=cadence, bounceresolution=20.0, dense_output=dense,
+                      max_steps_per_launch=budget)
         ens.set_guiding_centers(w["pos"], w["v"], pa=w["pa"], t0=0.5, mass=w["mass"], charge=w["charge"])
         ens.upload()
         st = ens.advance("gc", delta)
