@@ -141,10 +141,10 @@ def test_shared_between_warps(model, n, cadence, dense):
         w = dict(w, mass=np.full(n, W.m_pr), charge=np.full(n, W.e), v=np.linspace(3e5, 3e6, n), pos=W.config3(n, 2)["pos"])
     delta = np.random.default_rng(4).choice([0.0, 0.01, 0.03, 0.06], n)
     out = []
-    for budget in (0, 1 << 40):
+    for budget, graph in ((0, 0), (0, 1), (1 << 40, 0)):
         ens = Ensemble(MODELS[model](), n, max_rows=64)
         ens.configure(rtol=1e-7, atol=1e-7, gctimestep=cadence, bounceresolution=20.0, dense_output=dense,
-                      max_steps_per_launch=budget)
+                      max_steps_per_launch=budget, use_graph=graph)
         ens.set_guiding_centers(w["pos"], w["v"], pa=w["pa"], t0=0.5, mass=w["mass"], charge=w["charge"])
         ens.upload()
         st = ens.advance("gc", delta)
@@ -153,5 +153,31 @@ def test_shared_between_warps(model, n, cadence, dense):
         out.append([h[a].copy() for a in ("s", "t_row", "tcur", "mu", "status", "flags", "naccept", "nreject", "nfcn")] +
                    [nrows, np.where(np.arange(64)[None, :, None] < nrows[:, None, None], rows, 0.0),
                     np.array([st[a] for a in ("accepted", "rejected", "rhs_evals", "done", "failed")])])
-    for a, b in zip(*out):
+    for a, g, b in zip(*out):
         assert np.array_equal(a, b, equal_nan=a.dtype.kind == "f")
+        assert np.array_equal(g, b, equal_nan=a.dtype.kind == "f")
+
+
+def test_shared_rows_full_and_resume():
+    """A row buffer that fills up: the tracers stop and are resumed, shared or not."""
+    from rapt_gb300 import Ensemble
+    n = 9001
+    w = W.config2(n, seed=12)
+    delta = np.random.default_rng(5).choice([0.01, 0.03, 0.06], n)
+    out = []
+    for budget in (0, 1 << 40):
+        ens = Ensemble(F.DoubleDipole(), n, max_rows=4)
+        ens.configure(rtol=1e-7, atol=1e-7, gctimestep=0.01, max_steps_per_launch=budget)
+        ens.set_guiding_centers(w["pos"], w["v"], pa=w["pa"], t0=0.5, mass=w["mass"], charge=w["charge"])
+        ens.upload()
+        ens.advance("gc", delta)
+        got = []
+        for _ in range(4):
+            rows, _, nrows, _, _ = ens.rows()
+            got += [nrows, np.where(np.arange(4)[None, :, None] < nrows[:, None, None], rows, 0.0)]
+            ens.advance_resume("gc")
+        h = ens.download()
+        out.append(got + [h[a].copy() for a in ("s", "t_row", "status", "flags", "naccept", "nreject", "nfcn")])
+    assert (out[0][0] == 3).any() and out[0][2].any()  # a row and its possible switch row have to fit
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
