@@ -866,7 +866,7 @@ static int advance_impl(Ctx* c, int kind, const double* delta, double delta_all,
   // round): both end in a tail of a few long tracers, which then overlap instead
   // of following one another. 3,001 Adaptive tracers in the breathing dipole, plain
   // form: 30.0 ms one after the other, 16.3 ms side by side. The plain form now
-  // hands switched tracers over inside one launch (k_adaptive: 14.0 ms).
+  // hands switched tracers over inside one launch (k_adaptive: 12.3 ms).
   auto enqueue_round = [&](const DevEnsemble& Ev, int gp, int gg, int blk) -> int {
     CK(cudaMemsetAsync(c->scratch, 0, kRoundWords * sizeof(unsigned long long), s));
     LaunchArgs a{Ev, P, c->scratch, 0, blk, s};
