@@ -104,8 +104,9 @@ size_t ensemble_bytes(int64_t n, int max_rows, int max_sw) {
   size_t b = 0;
   b += 3 * al(N);                                      // mode, mode0, seg_active
   b += al(N * max_rows) + al(N * max_sw);              // row_mode, sw_mode
-  b += 7 * al(N * 4);                                  // status, flags, nrows, nswitch, nseg, ring[2]
+  b += 5 * al(N * 4);                                  // status, flags, nrows, nswitch, nseg
   b += 22 * al(N * 8);                                 // doubles
+  b += 2 * al(N * 8);                                  // ring[2]
   b += al(N * max_rows * 7 * 8) + al(N * max_sw * 8);  // rows, sw_time
   b += 3 * al(N * 8);                                  // int64 counters
   return b;
@@ -512,7 +513,7 @@ int rapt_ensemble_alloc(void* ctx, int64_t n, int32_t max_rows, int32_t max_swit
   E.nrows = carve<int32_t>(p, N);
   E.nswitch = carve<int32_t>(p, N);
   E.nseg = carve<int32_t>(p, N);
-  for (int i = 0; i < 2; ++i) E.ring[i] = carve<int32_t>(p, N);
+  for (int i = 0; i < 2; ++i) E.ring[i] = carve<unsigned long long>(p, N);
   E.t_int = carve<double>(p, N);
   E.t_row = carve<double>(p, N);
   E.tcur = carve<double>(p, N);
@@ -825,7 +826,7 @@ static int advance_impl(Ctx* c, int kind, const double* delta, double delta_all,
     const int bps_s = std::min(dense ? T.occ_gc_dense_share(block) : T.occ_gc_share(block), bps_g);
     grid_s = std::max(grid_of(bps_s, 32, block), std::min(bps_s, 1) * c->num_sms);
     const size_t warps = (size_t)grid_s * (block / 32);
-    share_head = (warps * (kMailWords + 1) * 4 + 255) / 256 * 256;
+    share_head = (warps * (kMailWords * 4 + 8) + 255) / 256 * 256;
     const size_t bytes = share_head + N * kMidWords * 8;
     if (grid_s > 0 && c->share_bytes < bytes) {
       cudaFree(c->share);
@@ -836,7 +837,7 @@ static int advance_impl(Ctx* c, int kind, const double* delta, double delta_all,
     }
     if (grid_s > 0) {
       E.mail = (int32_t*)c->share;
-      E.waitq = E.mail + warps * kMailWords;
+      E.waitq = (unsigned long long*)(E.mail + warps * kMailWords);
       E.mid = (double*)(c->share + share_head);
     }
   }
@@ -875,7 +876,7 @@ static int advance_impl(Ctx* c, int kind, const double* delta, double delta_all,
     else
       a.E.mode0 = Ev.mode;
     if (hand) {
-      for (int i = 0; i < 2; ++i) CK(cudaMemsetAsync(Ev.ring[i], 0, (size_t)Ev.n * 4, s));
+      for (int i = 0; i < 2; ++i) CK(cudaMemsetAsync(Ev.ring[i], 0, (size_t)Ev.n * 8, s));
       k_count_left<<<(unsigned)((Ev.n + 255) / 256), 256, 0, s>>>(Ev, c->scratch, false);
       CK(cudaGetLastError());
       a.grid = grid_a;

@@ -107,14 +107,14 @@ struct DevEnsemble {
   // longest expected work first); null: index order
   const int32_t* order;
   // hand-over rings of k_adaptive, n entries each ([mode]: tracers that switched to
-  // that mode, index + 1; 0: empty)
-  int32_t* ring[2];
+  // that mode; ring.cuh)
+  unsigned long long* ring[2];
   // sharing of tracers between the warps of a k_gc_share launch: state of tracers given
   // away inside an interval (kMidWords arrays of n), a mailbox of kMailWords a warp, and
   // the ring of the warps that wait (one entry a warp)
   double* mid;
   int32_t* mail;
-  int32_t* waitq;
+  unsigned long long* waitq;
 };
 constexpr int kMidWords = 9, kMailWords = 8;
 constexpr int kRoundWords = 10;  // words of Scratch that are reset for every round

@@ -21,6 +21,7 @@
 #pragma once
 #include "fieldline.cuh"
 #include "mlp.cuh"
+#include "ring.cuh"
 #include "rhs.cuh"
 #include "steppers.cuh"
 
@@ -267,27 +268,17 @@ __device__ __forceinline__ void warp_refill(unsigned long long* queue, const Dev
 
 // ---- hand-over between the two modes inside one launch (k_adaptive)
 // A tracer that switches is stored, fenced and put into the ring of its new mode;
-// a lane of that mode without a tracer takes it from there. A ring cannot run
-// over: it has n entries and a tracer is in at most one ring at a time. An entry
-// is published by its own store, so a taker sees only complete entries.
+// a lane of that mode without a tracer takes it from there (ring.cuh). A ring cannot
+// run over: it has n entries and a tracer is in at most one ring at a time.
 __device__ __forceinline__ void hand_over(const DevEnsemble& E, Scratch* S, int mode, int64_t idx) {
   __threadfence();
-  const unsigned long long at = atomicAdd(&S->ring_tail[mode], 1ull);
-  atomicExch(&E.ring[mode][at % (unsigned long long)E.n], (int32_t)idx + 1);
+  ring_put<Atomics>(E.ring[mode], (unsigned long long)E.n, &S->ring_tail[mode], (int32_t)idx);
 }
-__device__ __forceinline__ int64_t take_entry(int32_t* ring, unsigned long long entries, unsigned long long* head) {
-  for (int tries = 0; tries < 4; ++tries) {
-    const unsigned long long at = *(volatile unsigned long long*)head;
-    int32_t* e = &ring[at % entries];
-    const int32_t v = *(volatile int32_t*)e;
-    if (v == 0) return -1;
-    if (atomicCAS(head, at, at + 1) == at) {
-      atomicExch(e, 0);
-      __threadfence();
-      return (int64_t)v - 1;
-    }
-  }
-  return -1;
+__device__ __forceinline__ int64_t take_entry(unsigned long long* ring, unsigned long long entries,
+                                              unsigned long long* head) {
+  const int64_t v = ring_take<Atomics>(ring, entries, head);
+  if (v >= 0) __threadfence();
+  return v;
 }
 __device__ __forceinline__ int64_t take_over(const DevEnsemble& E, Scratch* S, int mode) {
   return take_entry(E.ring[mode], (unsigned long long)E.n, &S->ring_head[mode]);
@@ -333,8 +324,7 @@ __device__ __forceinline__ void share_wait(const DevEnsemble& E, Scratch* S, int
   const unsigned warps = gridDim.x * (blockDim.x >> 5), w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   int32_t* mail = E.mail + (size_t)w * kMailWords;
   if (lane == 0) {
-    const unsigned long long at = atomicAdd(&S->wait_tail, 1ull);
-    atomicExch(&E.waitq[at % warps], (int32_t)w + 1);
+    ring_put<Atomics>(E.waitq, warps, &S->wait_tail, (int32_t)w);
   }
   for (int poll = 0; poll < kPolls + 4096; ++poll) {
     int got = 0;
