@@ -760,8 +760,11 @@ static int advance_impl(Ctx* c, int kind, const double* delta, double delta_all,
   int block_g = block;
   if (f32 && kind == RAPT_KIND_GC && c->cfg.threads_per_block <= 0 && !c->cfg.per_tracer_launches)
     block_g = (int)std::min<int64_t>(1024, 128 * ((c->n + 128 * c->num_sms - 1) / (128 * (int64_t)c->num_sms)));
+  const bool collect = c->cfg.collect != 0;
+  if (block_g > block && T.occ_gc32_lrn[lrn](block_g, collect) < 1) block_g = block;  // no room for the samples' rows
   int bps_g = dense ? T.occ_gc_dense(block)
-                    : (tab != 0 ? T.occ_gc[tab](block) : (f32 ? T.occ_gc32_lrn[lrn](block_g) : T.occ_gc_lrn[lrn](block)));
+                    : (tab != 0 ? T.occ_gc[tab](block)
+                                : (f32 ? T.occ_gc32_lrn[lrn](block_g, collect) : T.occ_gc_lrn[lrn](block, collect)));
   if (c->cfg.blocks_per_sm > 0) {
     bps_p = std::min(bps_p, c->cfg.blocks_per_sm);
     bps_g = std::min(bps_g, c->cfg.blocks_per_sm);

@@ -77,14 +77,15 @@ int occ_particle32(int block) {
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_particle32<kM>, block, 0);
   return nb;
 }
-int occ_gc32(int block) {
+int occ_gc32(int block, bool) {
   int nb = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_gc32<kM>, block, 0);
   return nb;
 }
-// guiding-centre kernels with the step learner; dynamic shared memory per warp
-// (the occupancy is taken without collection; a collecting launch needs more
-// shared memory per block, and its surplus blocks start as others finish)
+// guiding-centre kernels with the step learner; dynamic shared memory per warp: the
+// network's buffers and, when samples are collected, their raw rows. k_gc32 in blocks of
+// 1,024 threads needs up to 96 KB a block (learned form, collecting), above the 48 KB
+// that a launch may ask for without the attribute.
 template <int LRN>
 size_t lrn_smem(int block, bool collect) {
   return (size_t)(block / 32) * StepLearner<LRN>::warp_words(collect) * sizeof(uint32_t);
@@ -100,15 +101,20 @@ cudaError_t launch_gc32_lrn(const LaunchArgs& a) {
   return cudaGetLastError();
 }
 template <int LRN>
-int occ_gc_lrn(int block) {
+int occ_gc_lrn(int block, bool collect) {
   int nb = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_gc<kM, 0, LRN>, block, lrn_smem<LRN>(block, false));
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_gc<kM, 0, LRN>, block, lrn_smem<LRN>(block, collect));
   return nb;
 }
 template <int LRN>
-int occ_gc32_lrn(int block) {
+int occ_gc32_lrn(int block, bool collect) {
   int nb = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_gc32<kM, LRN>, block, lrn_smem<LRN>(block, false));
+  const size_t most = lrn_smem<LRN>(1024, true);
+  if (cudaFuncSetAttribute(k_gc32<kM, LRN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most) != cudaSuccess) {
+    cudaGetLastError();
+    if (lrn_smem<LRN>(block, collect) > 48 * 1024) return 0;
+  }
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_gc32<kM, LRN>, block, lrn_smem<LRN>(block, collect));
   return nb;
 }
 cudaError_t field_eval(const FieldP& f, int what, int64_t n, const double* tpos, double* out, cudaStream_t s) {
@@ -175,13 +181,11 @@ void RAPT_CAT(register_model_, RAPT_MODEL)(ModelTable* t) {
   t->occ_gc[0] = occ_gc<0>;
   t->occ_gc[1] = occ_gc<1>;
   t->particle32 = launch_particle32;
-  t->gc32 = launch_gc32;
   t->occ_particle32 = occ_particle32;
-  t->occ_gc32 = occ_gc32;
   t->gc_lrn[0] = launch_gc<0>;
   t->gc_lrn[1] = launch_gc_lrn<1>;
   t->gc_lrn[2] = launch_gc_lrn<2>;
-  t->occ_gc_lrn[0] = occ_gc<0>;
+  t->occ_gc_lrn[0] = [](int block, bool) { return occ_gc<0>(block); };
   t->occ_gc_lrn[1] = occ_gc_lrn<1>;
   t->occ_gc_lrn[2] = occ_gc_lrn<2>;
   t->gc32_lrn[0] = launch_gc32;

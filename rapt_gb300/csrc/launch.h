@@ -30,6 +30,7 @@ inline int team_lanes(int64_t n, int sms, int model) {
 
 using LaunchFn = cudaError_t (*)(const LaunchArgs&);
 using OccFn = int (*)(int block);
+using OccLrnFn = int (*)(int block, bool collect);  // collect: with shared memory for samples
 using FieldEvalFn = cudaError_t (*)(const FieldP& f, int what, int64_t n, const double* tpos, double* out,
                                     cudaStream_t s);
 using RhsEvalFn = cudaError_t (*)(const KParams& P, int mode, int64_t n, const double* state, const double* mass,
@@ -56,12 +57,12 @@ struct ModelTable {
   LaunchFn gc[2];
   OccFn occ_particle[2];
   OccFn occ_gc[2];
-  LaunchFn particle32, gc32;  // FP32-stage form (DOP853 / DOPRI5)
-  OccFn occ_particle32, occ_gc32;
+  LaunchFn particle32;  // FP32-stage form (DOP853)
+  OccFn occ_particle32;
   // guiding-centre DOPRI5 kernels with the step learner: [0] plain, [1] sample
   // collection, [2] MLP proposals; FP64 and FP32-stage forms
   LaunchFn gc_lrn[3], gc32_lrn[3];
-  OccFn occ_gc_lrn[3], occ_gc32_lrn[3];
+  OccLrnFn occ_gc_lrn[3], occ_gc32_lrn[3];
   FieldEvalFn field_eval;
   RhsEvalFn rhs_eval;
   AdaptiveInitFn adaptive_init;
