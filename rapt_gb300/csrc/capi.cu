@@ -771,9 +771,11 @@ static int advance_impl(Ctx* c, int kind, const double* delta, double delta_all,
   }
   if (bps_p < 1 || bps_g < 1) return fail(c, RAPT_ERR_CUDA, "kernel does not fit on an SM");
   // Adaptive in the plain form: one grid for both modes, with hand-over (k_adaptive);
-  // it needs a block of each mode on an SM
+  // it needs a block of each mode on an SM. Not with a step budget: lanes that have spent
+  // theirs take nothing more, and the warps of the other mode would wait for tracers that
+  // nobody advances in this launch (0.4 s of polls a launch instead of a few ms).
   int bps_a = kind == RAPT_KIND_ADAPTIVE && form == RAPT_FORM_PLAIN && tab == 0 && !dense && lrn == 0 &&
-                      !c->cfg.per_tracer_launches
+                      !c->cfg.per_tracer_launches && c->cfg.max_steps_per_launch <= 0
                   ? T.occ_adaptive(block)
                   : 0;
   if (c->cfg.blocks_per_sm > 0) bps_a = std::min(bps_a, 2 * c->cfg.blocks_per_sm);

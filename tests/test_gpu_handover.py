@@ -49,3 +49,15 @@ def test_each_tracer_is_advanced_once(n, switching):
             assert np.array_equal(d[a], h[a]), a
         assert st["accepted"] == d["naccept"].sum() and st["switches"] == d["nswitch"].sum()
         assert st["done"] == n and st["failed"] == 0
+
+
+@pytest.mark.parametrize("cfg", [{}, {"blocks_per_sm": 1, "threads_per_block": 32}])
+def test_a_step_budget_bounds_a_launch(cfg):
+    """Several times as many tracers as a launch has lanes, and a budget of 100 attempts
+    a lane: a launch that leaves tracers to the next ends within some ms, without waits
+    (warps that wait in vain give up after 2^18 polls of a microsecond, 262 ms)."""
+    n = 60000 if cfg else 200000
+    which = np.arange(n) % 4096
+    st = _sheet(which, max_rows=256, max_steps_per_launch=100, **cfg).advance("adaptive", 20.0)
+    assert st["done"] == n and st["failed"] == 0
+    assert st["launches"] > 4 and st["kernel_ms"] < 60.0 * st["launches"], (st["kernel_ms"], st["launches"])
