@@ -802,7 +802,12 @@ static int advance_impl(Ctx* c, int kind, const double* delta, double delta_all,
   // have no teams: below 32 tracers a sub-partition a warp with fewer waits for fewer
   // other tracers' intervals (256 particles: kernel 7.2 -> 5.7 ms).
   P.lanes_p = f32 ? 32 : (int)std::max<int64_t>(1, std::min<int64_t>(32, (c->n + 4 * c->num_sms - 1) / (4 * c->num_sms)));
-  P.lanes_g = f32 || tab != 0 ? 32 : team_lanes(c->n, c->num_sms, c->field.model);
+  const bool can_share = kind == RAPT_KIND_GC && form == RAPT_FORM_PLAIN && tab == 0 && lrn == 0 &&
+                         !c->cfg.per_tracer_launches && c->cfg.max_steps_per_launch <= 0 &&
+                         !(dense && c->field.model == RAPT_GRID) && c->n <= 32ll * 32 * c->num_sms;
+  P.lanes_g = 32;
+  if (!f32 && tab == 0)
+    P.lanes_g = team_lanes(c->n, c->num_sms, c->field.model, can_share ? 1 : (kind == RAPT_KIND_GC ? 2 : 3));
   auto grid_of = [&](int bps, int lanes, int threads) {
     const int64_t warps = (c->n + lanes - 1) / lanes, blocks = (warps * 32 + threads - 1) / threads;
     return (int)std::min<int64_t>((int64_t)c->num_sms * bps, blocks);
@@ -824,9 +829,7 @@ static int advance_impl(Ctx* c, int kind, const double* delta, double delta_all,
   // intervals; without memory for it the plain kernel runs.
   int grid_s = 0;
   size_t share_head = 0;  // bytes of the mailboxes and the ring
-  if (kind == RAPT_KIND_GC && form == RAPT_FORM_PLAIN && tab == 0 && lrn == 0 && !c->cfg.per_tracer_launches &&
-      c->cfg.max_steps_per_launch <= 0 && P.lanes_g == 32 && !(dense && c->field.model == RAPT_GRID) &&
-      c->n <= 32ll * 32 * c->num_sms) {
+  if (can_share && P.lanes_g == 32) {
     // (no more blocks than the plain kernel's, which the field-line scratch is sized for)
     const int bps_s = std::min(dense ? T.occ_gc_dense_share(block) : T.occ_gc_share(block), bps_g);
     grid_s = std::max(grid_of(bps_s, 32, block), std::min(bps_s, 1) * c->num_sms);

@@ -18,13 +18,19 @@ struct LaunchArgs {
 // idle while the busy ones issue whole right-hand sides. Spread over one warp a
 // sub-partition, and no more to a warp than a round of teams serves (rhs.cuh: 4
 // tracers, 2 where a team is 16 lanes), they take a quarter of the FP64
-// instructions a warp; up to three rounds' worth a sub-partition that is less of
-// the pipe than one full warp's right-hand sides.
-inline int team_lanes(int64_t n, int sms, int model) {
+// instructions a warp. Up to `rounds` rounds' worth a sub-partition, that is; above, 32
+// a warp. Tracers that warps share among themselves (k_gc_share): one round, as they
+// spread by themselves (7,296 in the double dipole 3.9 -> 3.0 ms, 3,000 in the breathing
+// dipole 4.5 -> 3.0, 7,296 in the sheet 62 -> 55). Where they stay, two: at three, 7,296
+// in the double dipole take 3.99 ms, 32 a warp 3.65, and 3,000 in the breathing dipole
+// 4.59 and 3.91; at two, 4,864 and 2,432 take 2.69 and 3.40, 32 a warp 3.59 and 3.91.
+// Adaptive, where a launch's end is long: three (7,296 in the breathing dipole 22.5 ms,
+// 32 a warp 23.3; 3,648 11.7 and 22.9).
+inline int team_lanes(int64_t n, int sms, int model, int rounds) {
   const int64_t warps = 4LL * sms, per = (n + warps - 1) / warps;
   const bool timed = model == RAPT_VAR_EARTH_DIPOLE || model == RAPT_COMPRESSED_DIPOLE || model == RAPT_GRID;
   const int most = timed ? 2 : 4;
-  if (per > 3 * most) return 32;
+  if (per > rounds * most) return 32;
   return (int)(per < 1 ? 1 : (per > most ? most : per));
 }
 
