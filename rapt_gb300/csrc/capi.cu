@@ -754,12 +754,15 @@ static int advance_impl(Ctx* c, int kind, const double* delta, double delta_all,
   const bool dense = c->cfg.dense_output != 0;
   if (dense && kind != RAPT_KIND_PARTICLE && c->max_rows < 18)
     return fail(c, RAPT_ERR_INVALID, "dense output needs max_rows >= 18 (a step may cover 17 output times)");
-  // k_gc32 takes one block an SM, as large as the ensemble fills (its warps keep in
-  // step, fp32_kernels.cuh), unless a block size is asked for; in Adaptive rounds the
-  // particle kernel has to find room on the same SMs, and blocks stay small.
+  // k_gc32 takes one block an SM, as large as the ensemble fills, whose warps keep in
+  // step (fp32_kernels.cuh): from 512 threads on, below which a sub-partition has too few
+  // of the block's warps to gain. Not where a block size is asked for, nor in Adaptive
+  // rounds, where the particle kernel has to find room on the same SMs.
   int block_g = block;
-  if (f32 && kind == RAPT_KIND_GC && c->cfg.threads_per_block <= 0 && !c->cfg.per_tracer_launches)
-    block_g = (int)std::min<int64_t>(1024, 128 * ((c->n + 128 * c->num_sms - 1) / (128 * (int64_t)c->num_sms)));
+  if (f32 && kind == RAPT_KIND_GC && c->cfg.threads_per_block <= 0 && !c->cfg.per_tracer_launches) {
+    const int64_t fill = 128 * ((c->n + 128 * c->num_sms - 1) / (128 * (int64_t)c->num_sms));
+    if (fill >= 512) block_g = (int)std::min<int64_t>(1024, fill);
+  }
   const bool collect = c->cfg.collect != 0;
   if (block_g > block && T.occ_gc32_lrn[lrn](block_g, collect) < 1) block_g = block;  // no room for the samples' rows
   int bps_g = dense ? T.occ_gc_dense(block)
@@ -817,7 +820,8 @@ static int advance_impl(Ctx* c, int kind, const double* delta, double delta_all,
   const bool both = kind == RAPT_KIND_ADAPTIVE && !hand;
   const int grid_a = 2 * std::max(grid_of(bps_a / 2, P.lanes_p, block), grid_of(bps_a / 2, P.lanes_g, block));
   const int grid_p = grid_of(both ? (bps_p + 1) / 2 : bps_p, P.lanes_p, block);
-  const int grid_g = grid_of(both ? (bps_g + 1) / 2 : bps_g, P.lanes_g, block_g);
+  // blocks in step: one on every SM, over which the tracers are dealt out
+  const int grid_g = block_g > block ? c->num_sms * bps_g : grid_of(both ? (bps_g + 1) / 2 : bps_g, P.lanes_g, block_g);
 
   // Guiding centres in the plain form, from one warp a sub-partition up to 32: tracers
   // shared between the warps at the end of the launch (k_gc_share, k_gc_dense<M, true>).

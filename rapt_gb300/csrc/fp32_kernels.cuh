@@ -244,10 +244,10 @@ __global__ void __launch_bounds__(128, 2) k_particle32(DevEnsemble E, const __gr
 }
 
 // The warps of a block that share a sub-partition (warp index mod 4) and meet at a
-// barrier at every stage. Off (the warps go on by themselves) in blocks where a
-// sub-partition has only a few warps of the block.
+// barrier at every stage (ON). Off, the warps go on by themselves.
+template <bool ON>
 struct StageGroup {
-  bool on;
+  static constexpr bool on = ON;
   // whether any warp of the group has a tracer left: they stay together until none has
   __device__ __forceinline__ bool any(bool busy) const {
     if (!on) return busy;
@@ -267,7 +267,7 @@ struct StageGroup {
   }
 };
 
-template <int M, int LRN = 0>
+template <int M, int LRN, bool GROUP>
 // LRN: 0 plain controller, 1 training-sample collection, 2 MLP step proposals.
 // 64 registers, 32 warps an SM: the balance between resident warps (the float-float
 // stages are long dependent FP32 chains) and the local-memory traffic of spills
@@ -280,11 +280,13 @@ template <int M, int LRN = 0>
 // centres) and 153 -> 126 ms (learned, 1M). Measured on the same two: barriers once
 // an attempt 14.5 / 129; blocks of 512 (4 warps a group) 15.1 / 147, of 256
 // 15.9 / 154: the more warps share the fetches the better; two warps to a
-// sub-partition (blocks of 256) gain nothing and go on by themselves. The warps' first
-// tracers are dealt out over the blocks: taken by arrival, one block had the longest
-// 1,024 of an ensemble that fills the GPU once (150,000 guiding centres 18.9 -> 20.0 ms
-// by arrival, 17.9 dealt out).
-__global__ void __launch_bounds__(1024, 1) k_gc32(DevEnsemble E, const __grid_constant__ KParams P, Scratch* S) {
+// sub-partition gain nothing, so below 512 threads to fill an SM, in Adaptive rounds and
+// where a block size is asked for, blocks of up to 128 run without groups (GROUP false).
+// The warps' first tracers are dealt out over the blocks, one on every SM: taken by
+// arrival, one block had the longest 1,024 of an ensemble that fills the GPU once
+// (150,000 guiding centres 18.9 -> 20.0 ms by arrival, 17.9 dealt out).
+__global__ void __launch_bounds__(GROUP ? 1024 : 128, GROUP ? 1 : 8)
+    k_gc32(DevEnsemble E, const __grid_constant__ KParams P, Scratch* S) {
   int64_t idx = -1;
   bool exhausted = false;
   long long budget = P.budget;
@@ -369,9 +371,9 @@ __global__ void __launch_bounds__(1024, 1) k_gc32(DevEnsemble E, const __grid_co
   };
 
   for (;;) {
-    warp_refill(&S->queue[1], E, RAPT_MODE_GC, 32, idx, exhausted, load, &dealt);
+    warp_refill(&S->queue[1], E, RAPT_MODE_GC, 32, idx, exhausted, load, GROUP ? &dealt : nullptr);
     const bool busy = !__all_sync(kFull, idx < 0);
-    const StageGroup group{blockDim.x >= 512 && blockDim.x % 128 == 0};
+    const StageGroup<GROUP> group{};
     if (!group.any(busy)) break;
     lr.infer(P, h);
 
@@ -451,15 +453,20 @@ __global__ void __launch_bounds__(1024, 1) k_gc32(DevEnsemble E, const __grid_co
     DF y1[4], k7[4];
     double err = 0.0;
     // in a group all lanes of a warp with an attempt to make go through it, and the
-    // group's other warps meet it at the stages; by itself a lane without a tracer stays
-    // out (its zeros would take the slow paths of divisions: 7 guiding centres 1.9 -> 2.5 ms)
-    const bool any_attempt = __any_sync(kFull, attempt);
-    if (group.on ? any_attempt : attempt) {
+    // group's other warps meet it at the stages; without, the attempt is part of the branch
+    // below: a lane without a tracer stays out (its zeros would take the slow paths of
+    // divisions: 7 guiding centres 1.9 -> 2.5 ms), and apart from the branch it spills more
+    // (262,144 in blocks of 128: 10.1 ms, 8.45 so)
+    auto dopri5 = [&]() {
       dopri5_attempt_df_rolled<4>(rhs, rt, y, k1, h, scale[3], P.rtol, P.atol, y1, k7, err, group);
-    } else {
-      for (int s = 0; s < 6; ++s) group();
+    };
+    if (GROUP) {
+      if (__any_sync(kFull, attempt)) dopri5();
+      else
+        for (int s = 0; s < 6; ++s) group();
     }
     if (attempt) {
+      if (!GROUP) dopri5();
       nfcn += 6;
       st.rhs += 6;
       lr.on_attempt(P, h, err, last);

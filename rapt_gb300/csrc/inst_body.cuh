@@ -68,18 +68,9 @@ cudaError_t launch_particle32(const LaunchArgs& a) {
   k_particle32<kM><<<a.grid, a.block, 0, a.stream>>>(a.E, a.P, a.S);
   return cudaGetLastError();
 }
-cudaError_t launch_gc32(const LaunchArgs& a) {
-  k_gc32<kM><<<a.grid, a.block, 0, a.stream>>>(a.E, a.P, a.S);
-  return cudaGetLastError();
-}
 int occ_particle32(int block) {
   int nb = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_particle32<kM>, block, 0);
-  return nb;
-}
-int occ_gc32(int block, bool) {
-  int nb = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_gc32<kM>, block, 0);
   return nb;
 }
 // guiding-centre kernels with the step learner; dynamic shared memory per warp: the
@@ -95,9 +86,12 @@ cudaError_t launch_gc_lrn(const LaunchArgs& a) {
   k_gc<kM, 0, LRN><<<a.grid, a.block, lrn_smem<LRN>(a.block, a.P.collect != 0), a.stream>>>(a.E, a.P, a.S);
   return cudaGetLastError();
 }
+// blocks of more than 128 threads are those whose warps keep in step
 template <int LRN>
-cudaError_t launch_gc32_lrn(const LaunchArgs& a) {
-  k_gc32<kM, LRN><<<a.grid, a.block, lrn_smem<LRN>(a.block, a.P.collect != 0), a.stream>>>(a.E, a.P, a.S);
+cudaError_t launch_gc32(const LaunchArgs& a) {
+  const size_t smem = lrn_smem<LRN>(a.block, a.P.collect != 0);
+  if (a.block > 128) k_gc32<kM, LRN, true><<<a.grid, a.block, smem, a.stream>>>(a.E, a.P, a.S);
+  else k_gc32<kM, LRN, false><<<a.grid, a.block, smem, a.stream>>>(a.E, a.P, a.S);
   return cudaGetLastError();
 }
 template <int LRN>
@@ -107,14 +101,20 @@ int occ_gc_lrn(int block, bool collect) {
   return nb;
 }
 template <int LRN>
-int occ_gc32_lrn(int block, bool collect) {
+int occ_gc32(int block, bool collect) {
   int nb = 0;
-  const size_t most = lrn_smem<LRN>(1024, true);
-  if (cudaFuncSetAttribute(k_gc32<kM, LRN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most) != cudaSuccess) {
-    cudaGetLastError();
-    if (lrn_smem<LRN>(block, collect) > 48 * 1024) return 0;
+  const size_t smem = lrn_smem<LRN>(block, collect);
+  if (block <= 128) {
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_gc32<kM, LRN, false>, block, smem);
+    return nb;
   }
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_gc32<kM, LRN>, block, lrn_smem<LRN>(block, collect));
+  const cudaError_t e = cudaFuncSetAttribute(k_gc32<kM, LRN, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)lrn_smem<LRN>(1024, true));
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    if (smem > 48 * 1024) return 0;
+  }
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_gc32<kM, LRN, true>, block, smem);
   return nb;
 }
 cudaError_t field_eval(const FieldP& f, int what, int64_t n, const double* tpos, double* out, cudaStream_t s) {
@@ -188,12 +188,12 @@ void RAPT_CAT(register_model_, RAPT_MODEL)(ModelTable* t) {
   t->occ_gc_lrn[0] = [](int block, bool) { return occ_gc<0>(block); };
   t->occ_gc_lrn[1] = occ_gc_lrn<1>;
   t->occ_gc_lrn[2] = occ_gc_lrn<2>;
-  t->gc32_lrn[0] = launch_gc32;
-  t->gc32_lrn[1] = launch_gc32_lrn<1>;
-  t->gc32_lrn[2] = launch_gc32_lrn<2>;
-  t->occ_gc32_lrn[0] = occ_gc32;
-  t->occ_gc32_lrn[1] = occ_gc32_lrn<1>;
-  t->occ_gc32_lrn[2] = occ_gc32_lrn<2>;
+  t->gc32_lrn[0] = launch_gc32<0>;
+  t->gc32_lrn[1] = launch_gc32<1>;
+  t->gc32_lrn[2] = launch_gc32<2>;
+  t->occ_gc32_lrn[0] = occ_gc32<0>;
+  t->occ_gc32_lrn[1] = occ_gc32<1>;
+  t->occ_gc32_lrn[2] = occ_gc32<2>;
   t->field_eval = field_eval;
   t->rhs_eval = rhs_eval;
   t->adaptive_init = adaptive_init;
