@@ -804,7 +804,6 @@ __device__ __forceinline__ void gc_body(const DevEnsemble& E, const KParams& P, 
     if (HAND) warp_take(E, S, RAPT_MODE_GC, P.lanes_g, idx, exhausted, spent, load);
     if (__all_sync(kFull, idx < 0)) break;
     lr.infer(P, h);
-    if (TAB != 0 && idx < 0) continue;  // RKF45 has no teams: a lane without a tracer stays out
 
     const GcRHS<M> rhs{P.f, charge, qinv, mu, minv, kmu, inv_mc, igv, gmv, gmv2, P.gc_eom, P.enforce_eq != 0};
 
@@ -942,7 +941,7 @@ __device__ __forceinline__ void gc_body(const DevEnsemble& E, const KParams& P, 
           h = hnew;
         }
       }
-    } else {
+    } else if (idx >= 0) {
       if (!(rt < xend)) { ended = true; }
       else if (nst > 1000000) { ended = true; fail = RAPT_ST_MAXSTEPS; }
       else {
