@@ -227,15 +227,24 @@ __global__ void k_prepare(DevEnsemble E, const double* delta, double delta_all, 
   E.t_int[k] = E.t_row[k];
 }
 
-// Start of a k_adaptive or k_gc_share launch: the tracers still to be advanced, counted.
-__global__ void k_count_left(DevEnsemble E, Scratch* S, bool gc_only) {
+// Start of a round: the tracers still to be advanced, counted. count: in_mode only
+// (Adaptive rounds of two kernels), or also pending and remaining of a k_adaptive launch
+// or, for guiding centres, of a k_gc_share launch.
+enum { kCountModes, kCountAll, kCountGc };
+__global__ void k_count_left(DevEnsemble E, Scratch* S, int count) {
   const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const bool left = k < E.n && !(E.flags[k] & RAPT_FLAG_DONE) && E.status[k] != RAPT_ST_ROWS_FULL &&
-                    (!gc_only || E.mode[k] == RAPT_MODE_GC);
+  const bool left = k < E.n && !(E.flags[k] & RAPT_FLAG_DONE) && E.status[k] != RAPT_ST_ROWS_FULL;
+  const bool gc = left && E.mode[k] == RAPT_MODE_GC;
+  const unsigned long long g = (unsigned long long)__syncthreads_count(gc);
   const unsigned long long c = (unsigned long long)__syncthreads_count(left);
   if (threadIdx.x == 0 && c) {
-    atomicAdd(&S->pending, c);
-    atomicAdd(&S->remaining, c);
+    if (g) atomicAdd(&S->in_mode[RAPT_MODE_GC], g);
+    if (c > g) atomicAdd(&S->in_mode[RAPT_MODE_PARTICLE], c - g);
+    const unsigned long long t = count == kCountGc ? g : c;
+    if (count != kCountModes && t) {
+      atomicAdd(&S->pending, t);
+      atomicAdd(&S->remaining, t);
+    }
   }
 }
 
@@ -816,12 +825,17 @@ static int advance_impl(Ctx* c, int kind, const double* delta, double delta_all,
     return (int)std::min<int64_t>((int64_t)c->num_sms * bps, blocks);
   };
   const bool hand = bps_a >= 2;
-  // otherwise an Adaptive round's two kernels run side by side: each takes half of the SMs' blocks
+  // otherwise an Adaptive round's two kernels run side by side (surplus_block)
   const bool both = kind == RAPT_KIND_ADAPTIVE && !hand;
+  if (both && !c->cfg.per_tracer_launches) {
+    P.full[RAPT_MODE_PARTICLE] = c->num_sms * bps_p;
+    P.full[RAPT_MODE_GC] = c->num_sms * bps_g;
+    P.grow = f32 ? 1 : 4;
+  }
   const int grid_a = 2 * std::max(grid_of(bps_a / 2, P.lanes_p, block), grid_of(bps_a / 2, P.lanes_g, block));
-  const int grid_p = grid_of(both ? (bps_p + 1) / 2 : bps_p, P.lanes_p, block);
+  const int grid_p = grid_of(bps_p, P.lanes_p, block);
   // blocks in step: one on every SM, over which the tracers are dealt out
-  const int grid_g = block_g > block ? c->num_sms * bps_g : grid_of(both ? (bps_g + 1) / 2 : bps_g, P.lanes_g, block_g);
+  const int grid_g = block_g > block ? c->num_sms * bps_g : grid_of(bps_g, P.lanes_g, block_g);
 
   // Guiding centres in the plain form, from one warp a sub-partition up to 32: tracers
   // shared between the warps at the end of the launch (k_gc_share, k_gc_dense<M, true>).
@@ -889,7 +903,7 @@ static int advance_impl(Ctx* c, int kind, const double* delta, double delta_all,
       a.E.mode0 = Ev.mode;
     if (hand) {
       for (int i = 0; i < 2; ++i) CK(cudaMemsetAsync(Ev.ring[i], 0, (size_t)Ev.n * 8, s));
-      k_count_left<<<(unsigned)((Ev.n + 255) / 256), 256, 0, s>>>(Ev, c->scratch, false);
+      k_count_left<<<(unsigned)((Ev.n + 255) / 256), 256, 0, s>>>(Ev, c->scratch, kCountAll);
       CK(cudaGetLastError());
       a.grid = grid_a;
       CK(T.adaptive(a));
@@ -898,7 +912,7 @@ static int advance_impl(Ctx* c, int kind, const double* delta, double delta_all,
     }
     if (grid_s > 0) {
       CK(cudaMemsetAsync(Ev.mail, 0, share_head, s));
-      k_count_left<<<(unsigned)((Ev.n + 255) / 256), 256, 0, s>>>(Ev, c->scratch, true);
+      k_count_left<<<(unsigned)((Ev.n + 255) / 256), 256, 0, s>>>(Ev, c->scratch, kCountGc);
       CK(cudaGetLastError());
       a.grid = grid_s;
       CK(dense ? T.gc_dense_share(a) : T.gc_share(a));
@@ -906,6 +920,11 @@ static int advance_impl(Ctx* c, int kind, const double* delta, double delta_all,
       return RAPT_OK;
     }
     if (both) {
+      if (P.full[0]) {
+        k_count_left<<<(unsigned)((Ev.n + 255) / 256), 256, 0, s>>>(Ev, c->scratch, kCountModes);
+        CK(cudaGetLastError());
+        ++kl;
+      }
       CK(cudaEventRecord(c->fork, s));
       CK(cudaStreamWaitEvent(c->side, c->fork, 0));
       a.stream = c->side;

@@ -48,6 +48,7 @@ struct KParams {
   long long budget;        // RK step attempts per thread per launch
   int max_rows, max_sw;    // per-tracer output capacity
   int max_segments;        // Adaptive: cap on advance() calls per tracer
+  int full[2], grow;       // Adaptive rounds: blocks of each mode's kernel that fill the GPU (surplus_block)
   int lanes_p, lanes_g;    // tracers a warp of the particle / guiding-centre kernel holds at a time (0: 32)
   // step-size MLP (learned forms) and training-sample collection
   const uint32_t* mlp_w;   // packed BF16 weights
@@ -117,7 +118,7 @@ struct DevEnsemble {
   unsigned long long* waitq;
 };
 constexpr int kMidWords = 9, kMailWords = 8;
-constexpr int kRoundWords = 10;  // words of Scratch that are reset for every round
+constexpr int kRoundWords = 12;  // words of Scratch that are reset for every round
 
 // Scratch words used by the persistent kernels (one block of device memory).
 struct Scratch {
@@ -128,6 +129,7 @@ struct Scratch {
   unsigned long long remaining;
   unsigned long long ring_head[2], ring_tail[2];
   unsigned long long wait_head, wait_tail;  // k_gc_share: positions in the ring of waiting warps
+  unsigned long long in_mode[2];  // Adaptive: tracers to advance at the round's start, by mode
   unsigned long long accepted, rejected, rhs, switches, done, failed;
 };
 

@@ -28,6 +28,7 @@ constexpr int kDenseSpan = 16;
 // row every 0.01 s: a pass 12.5 -> 12.0 ms, of which the kernel is some 7.
 template <int M, bool SHARE>
 __global__ void __launch_bounds__(128) k_gc_dense(DevEnsemble E, const __grid_constant__ KParams P, Scratch* S) {
+  if (!SHARE && surplus_block(P, S, RAPT_MODE_GC)) return;
   int64_t idx = -1;
   bool exhausted = false;
   long long budget = P.budget;

@@ -16,6 +16,7 @@ template <int M>
 // 4: 1.18e8, 6: 1.05e8, 8: 1.02e8).
 __global__ void __launch_bounds__(128, 2) k_particle32(DevEnsemble E, const __grid_constant__ KParams P,
                                                        Scratch* S) {
+  if (surplus_block(P, S, RAPT_MODE_PARTICLE)) return;
   int64_t idx = -1;
   bool exhausted = false;
   long long budget = P.budget;
@@ -287,6 +288,7 @@ template <int M, int LRN, bool GROUP>
 // (150,000 guiding centres 18.9 -> 20.0 ms by arrival, 17.9 dealt out).
 __global__ void __launch_bounds__(GROUP ? 1024 : 128, GROUP ? 1 : 8)
     k_gc32(DevEnsemble E, const __grid_constant__ KParams P, Scratch* S) {
+  if (!GROUP && surplus_block(P, S, RAPT_MODE_GC)) return;
   int64_t idx = -1;
   bool exhausted = false;
   long long budget = P.budget;

@@ -222,6 +222,34 @@ struct LaneStats {
   }
 };
 
+// Whether this block leaves the round to others. In an Adaptive round the particle and
+// the guiding-centre kernel run side by side, each with a grid that would fill the GPU,
+// of which half the blocks work: both kernels end in tails of few tracers, which overlap.
+// Where one mode has tracers for more than `grow` times its half and the other fewer than
+// for its own, the other gets the blocks that they take and the larger the rest. With
+// half whatever there was to do, 262,144 FP32-form electrons that all stay guiding
+// centres took 62 ms, the kernels one after the other 35 and 35 so; with full grids side
+// by side 262,144 protons in the sheet 740 ms for 440, as one kernel's long tail kept the
+// other off the GPU. grow (capi.cu): 1 in the FP32 forms, which need the warps; 4 in
+// FP64, where half the blocks nearly fill the pipe and fewer tracers an SM end sooner
+// (32,768 with dense rows 24.4 ms on half, 31.2 on all).
+__device__ __forceinline__ bool surplus_block(const KParams& P, const Scratch* S, int mode) {
+  if (P.full[0] == 0) return false;
+  float need[2];
+#pragma unroll
+  for (int m = 0; m < 2; ++m) {
+    const int lanes = m == RAPT_MODE_GC ? P.lanes_g : P.lanes_p;
+    need[m] = ceilf((float)S->in_mode[m] * 32.f / (float)(lanes * (int)blockDim.x));
+  }
+  const float mine = 0.5f * (float)P.full[mode], other = 0.5f * (float)P.full[1 - mode];
+  float take = ceilf(mine);
+  if (need[1 - mode] < other && need[mode] > (float)P.grow * mine)
+    take = ceilf(mine * (2.f - need[1 - mode] / other));
+  else if (need[mode] < mine && need[1 - mode] > (float)P.grow * other)
+    take = need[mode];
+  return (float)blockIdx.x >= take;
+}
+
 // Warp-wide refill: every lane without a tracer takes the next queue index
 // until it holds a tracer of this kernel's mode (as of the start of the round)
 // or the queue is exhausted.
@@ -684,6 +712,7 @@ __device__ __forceinline__ void particle_body(const DevEnsemble& E, const KParam
 
 template <int M, int TAB>
 __global__ void __launch_bounds__(128) k_particle(DevEnsemble E, const __grid_constant__ KParams P, Scratch* S) {
+  if (surplus_block(P, S, RAPT_MODE_PARTICLE)) return;
   particle_body<M, TAB, false>(E, P, S);
 }
 
@@ -1029,6 +1058,7 @@ __device__ __forceinline__ void gc_body(const DevEnsemble& E, const KParams& P, 
 
 template <int M, int TAB, int LRN = 0>
 __global__ void __launch_bounds__(128) k_gc(DevEnsemble E, const __grid_constant__ KParams P, Scratch* S) {
+  if (surplus_block(P, S, RAPT_MODE_GC)) return;
   gc_body<M, TAB, LRN, false, false>(E, P, S);
 }
 
