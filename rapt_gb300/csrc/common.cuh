@@ -118,7 +118,7 @@ struct DevEnsemble {
   unsigned long long* waitq;
 };
 constexpr int kMidWords = 9, kMailWords = 8;
-constexpr int kRoundWords = 12;  // words of Scratch that are reset for every round
+constexpr int kRoundWords = 14;  // words of Scratch that are reset for every round
 
 // Scratch words used by the persistent kernels (one block of device memory).
 struct Scratch {
@@ -130,6 +130,7 @@ struct Scratch {
   unsigned long long ring_head[2], ring_tail[2];
   unsigned long long wait_head, wait_tail;  // k_gc_share: positions in the ring of waiting warps
   unsigned long long in_mode[2];  // Adaptive: tracers to advance at the round's start, by mode
+  unsigned long long gone[2];     // k_adaptive: warps of either mode that have left the launch
   unsigned long long accepted, rejected, rhs, switches, done, failed;
 };
 

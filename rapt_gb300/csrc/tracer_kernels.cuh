@@ -316,36 +316,72 @@ __device__ __forceinline__ void retire(Scratch* S, bool finished) {
   atomicAdd(&S->remaining, ~0ull);
   if (finished) atomicAdd(&S->pending, ~0ull);
 }
+// Pause between two polls: a microsecond at first, for hand-overs that follow one
+// another, then 20, for launches of seconds.
+__device__ __forceinline__ void poll_pause(int poll) { __nanosleep(poll < 4096 ? 1000 : 20000); }
 // Lanes that the work queue no longer feeds take switched tracers. A warp with no
-// tracer at all waits for one, until every tracer of the launch has stopped or
-// kPolls polls of about a microsecond have passed (what is left then goes to the
-// next launch); the waited-for lanes are blocks of the same launch.
-constexpr int kPolls = 1 << 18;
+// tracer at all waits for one (blocks of the same launch hand them over), until every
+// tracer of the launch has stopped, or the other mode's warps (`others`) have all left
+// and nobody can hand one over any more, or kPolls polls, some 20 s, have passed; what is
+// left then goes to the next launch. (At 2^18 polls of a microsecond the warps of a mode
+// that had nothing to do for 0.3 s were gone for the rest of the launch.)
+constexpr int kPolls = 1 << 20;
 template <class LoadFn>
-__device__ __forceinline__ void warp_take(const DevEnsemble& E, Scratch* S, int mode, int lanes, int64_t& idx,
-                                          bool exhausted, bool spent, LoadFn&& load) {
+__device__ __forceinline__ void warp_take(const DevEnsemble& E, Scratch* S, int mode, int lanes, unsigned others,
+                                          int64_t& idx, bool exhausted, LoadFn&& load) {
   const int lane = threadIdx.x & 31;
-  const bool wants = exhausted && !spent && (lanes <= 0 || lane < lanes);
+  const bool wants = exhausted && (lanes <= 0 || lane < lanes);
+  bool last_look = false;
   for (int poll = 0; poll < kPolls; ++poll) {
     if (idx < 0 && wants) {
       idx = take_over(E, S, mode);
       if (idx >= 0) load(idx);
     }
     if (__any_sync(kFull, idx >= 0)) return;
-    if (!__any_sync(kFull, wants)) return;
-    unsigned long long left = 0;
-    if (lane == 0) left = *(volatile unsigned long long*)&S->remaining;
-    if (__shfl_sync(kFull, left, 0) == 0ull) return;
-    __nanosleep(1000);
+    if (last_look || !__any_sync(kFull, wants)) return;
+    int stop = 0;
+    if (lane == 0)
+      stop = *(volatile unsigned long long*)&S->remaining == 0ull
+                 ? 2
+                 : (int)(*(volatile unsigned long long*)&S->gone[1 - mode] >= (unsigned long long)others);
+    stop = __shfl_sync(kFull, stop, 0);
+    if (stop == 2) return;
+    last_look = stop == 1;  // what they handed over before they left is in the ring by now
+    if (!last_look) poll_pause(poll);
   }
+}
+// A warp of `mode` leaves a k_adaptive launch.
+__device__ __forceinline__ void warp_leaves(Scratch* S, int mode) {
+  __syncwarp();
+  if ((threadIdx.x & 31) == 0) {
+    __threadfence();
+    atomicAdd(&S->gone[mode], 1ull);
+  }
+}
+// Blocks of a k_adaptive launch that run particles; the rest run guiding centres. Half,
+// as either mode may get any number of tracers, unless one mode starts with more than four
+// times its half's and the other with fewer than its own: the other then gets the blocks
+// that its tracers take and an eighth of the grid at least, for those that switch.
+// 262,144 electrons that all stay guiding centres: half 174 ms, seven eighths 149 (k_gc
+// after an empty k_particle, at the full grid, 163).
+__device__ __forceinline__ unsigned particle_blocks(const KParams& P, const Scratch* S) {
+  const float half = 0.5f * (float)gridDim.x;
+  const float np = ceilf((float)S->in_mode[RAPT_MODE_PARTICLE] * 32.f / (float)(P.lanes_p * (int)blockDim.x));
+  const float ng = ceilf((float)S->in_mode[RAPT_MODE_GC] * 32.f / (float)(P.lanes_g * (int)blockDim.x));
+  const float least = fmaxf(1.f, floorf(0.25f * half));
+  float b = floorf(half);
+  if (np < half && ng > 4.f * half) b = fmaxf(np, least);
+  if (ng < half && np > 4.f * half) b = (float)gridDim.x - fmaxf(ng, least);
+  return (unsigned)b;
 }
 
 // ---- sharing of tracers between the warps of a launch (k_gc_share)
 // A warp without a tracer enters the ring of waiting warps and polls its mailbox,
 // until a warp with many tracers gives it some, every tracer of the launch has stopped
-// or kPolls polls (1 us each at first, then 20) have passed; it then closes its mailbox.
+// or kSharePolls polls, some 5 s, have passed; it then closes its mailbox.
 // Mailbox word 0: 0 open, -1 closed, -2 being filled, > 0 that many tracers in words 1..
 // All 32 lanes call these.
+constexpr int kSharePolls = 1 << 18;
 template <class LoadFn>
 __device__ __forceinline__ void share_wait(const DevEnsemble& E, Scratch* S, int64_t& idx, LoadFn&& load) {
   const int lane = threadIdx.x & 31;
@@ -354,11 +390,11 @@ __device__ __forceinline__ void share_wait(const DevEnsemble& E, Scratch* S, int
   if (lane == 0) {
     ring_put<Atomics>(E.waitq, warps, &S->wait_tail, (int32_t)w);
   }
-  for (int poll = 0; poll < kPolls + 4096; ++poll) {
+  for (int poll = 0; poll < kSharePolls + 4096; ++poll) {
     int got = 0;
     if (lane == 0) {
       got = *(volatile int32_t*)mail;
-      if (got == 0 && (poll >= kPolls || *(volatile unsigned long long*)&S->remaining == 0ull))
+      if (got == 0 && (poll >= kSharePolls || *(volatile unsigned long long*)&S->remaining == 0ull))
         got = atomicCAS(mail, 0, -1) == 0 ? -1 : 0;
     }
     got = __shfl_sync(kFull, got, 0);
@@ -373,7 +409,7 @@ __device__ __forceinline__ void share_wait(const DevEnsemble& E, Scratch* S, int
       __syncwarp();
       return;
     }
-    __nanosleep(poll < 4096 ? 1000 : 20000);
+    poll_pause(poll);
   }
 }
 // A warp with more tracers than a round of TEAMS teams serves gives them to waiting
@@ -435,9 +471,9 @@ __device__ __forceinline__ void put_row(const DevEnsemble& E, const KParams& P, 
 // HAND: part of k_adaptive (switched tracers are handed over instead of left to
 // the next round).
 template <int M, int TAB, bool HAND>
-__device__ __forceinline__ void particle_body(const DevEnsemble& E, const KParams& P, Scratch* S) {
+__device__ __forceinline__ void particle_body(const DevEnsemble& E, const KParams& P, Scratch* S, unsigned others = 0) {
   int64_t idx = -1;
-  bool exhausted = false, spent = false;
+  bool exhausted = false;
   long long budget = P.budget;
   LaneStats st;
 
@@ -502,7 +538,7 @@ __device__ __forceinline__ void particle_body(const DevEnsemble& E, const KParam
 
   for (;;) {
     warp_refill(&S->queue[0], E, RAPT_MODE_PARTICLE, P.lanes_p, idx, exhausted, load);
-    if (HAND) warp_take(E, S, RAPT_MODE_PARTICLE, P.lanes_p, idx, exhausted, spent, load);
+    if (HAND) warp_take(E, S, RAPT_MODE_PARTICLE, P.lanes_p, others, idx, exhausted, load);
     if (__all_sync(kFull, idx < 0)) break;
     if (idx < 0) continue;
 
@@ -536,7 +572,7 @@ __device__ __forceinline__ void particle_body(const DevEnsemble& E, const KParam
       if (budget <= 0) {
         store(idx, true);
         idx = -1;
-        exhausted = spent = true;
+        exhausted = true;
         if (HAND) retire(S, false);
         else st.pend++;
         continue;
@@ -707,6 +743,7 @@ __device__ __forceinline__ void particle_body(const DevEnsemble& E, const KParam
       idx = -1;
     }
   }
+  if (HAND) warp_leaves(S, RAPT_MODE_PARTICLE);
   st.flush(S);
 }
 
@@ -722,12 +759,12 @@ __global__ void __launch_bounds__(128) k_particle(DevEnsemble E, const __grid_co
 // (a proposal replaces the controller's next step after an accepted step and
 // HINIT at the next interval; a rejected proposal falls back to the controller).
 template <int M, int TAB, int LRN, bool HAND, bool SHARE>
-__device__ __forceinline__ void gc_body(const DevEnsemble& E, const KParams& P, Scratch* S) {
+__device__ __forceinline__ void gc_body(const DevEnsemble& E, const KParams& P, Scratch* S, unsigned others = 0) {
   static_assert(LRN == 0 || TAB == 0, "the step learner drives the DOPRI5 controller");
   static_assert(!SHARE || (TAB == 0 && LRN == 0 && !HAND), "sharing: the plain DOPRI5 form");
   constexpr bool COUNT = HAND || SHARE;  // tracers that stop are counted as they do
   int64_t idx = -1;
-  bool exhausted = false, spent = false;
+  bool exhausted = false;
   long long budget = P.budget;
   LaneStats st;
   StepLearner<LRN> lr;
@@ -830,7 +867,7 @@ __device__ __forceinline__ void gc_body(const DevEnsemble& E, const KParams& P, 
       if (__all_sync(kFull, idx < 0)) share_wait(E, S, idx, load);
       else share_give<GcTeam<M>::kTeams, GcTeam<M>::kMaxLanes>(E, S, idx, in_interval, store_mid);
     }
-    if (HAND) warp_take(E, S, RAPT_MODE_GC, P.lanes_g, idx, exhausted, spent, load);
+    if (HAND) warp_take(E, S, RAPT_MODE_GC, P.lanes_g, others, idx, exhausted, load);
     if (__all_sync(kFull, idx < 0)) break;
     lr.infer(P, h);
 
@@ -865,7 +902,7 @@ __device__ __forceinline__ void gc_body(const DevEnsemble& E, const KParams& P, 
       if (start && budget <= 0) {
         store(idx, true);
         idx = -1;
-        exhausted = spent = true;
+        exhausted = true;
         if (COUNT) retire(S, false);
         else st.pend++;
         start = false;
@@ -1053,6 +1090,7 @@ __device__ __forceinline__ void gc_body(const DevEnsemble& E, const KParams& P, 
       }
     }
   }
+  if (HAND) warp_leaves(S, RAPT_MODE_GC);
   st.flush(S);
 }
 
@@ -1077,9 +1115,9 @@ __global__ void __launch_bounds__(128) k_gc_share(DevEnsemble E, const __grid_co
 }
 
 // ---------------------------------------------------------------- Adaptive in one launch
-// Both modes in one grid (plain FP64 form): the first half of the blocks runs
-// particles, the second half guiding centres, and a tracer that switches is handed
-// to the other half at once. With a launch pair per round of switches, every round
+// Both modes in one grid (plain FP64 form): the first blocks run particles, half of
+// the grid mostly (particle_blocks), the others guiding centres, and a tracer that
+// switches is handed to the others at once. With a launch pair per round of switches, every round
 // ended in a tail of its longest segments (1.6-1.9 of 32 lanes active in most
 // rounds of the Harris sheet) while the tracers that had switched waited; here the
 // longest tracer alone sets the end. 32,768 Adaptive protons in the Harris sheet:
@@ -1087,8 +1125,9 @@ __global__ void __launch_bounds__(128) k_gc_share(DevEnsemble E, const __grid_co
 // 14.0 ms (41.0 and 12.3 with the particle controller as it is now).
 template <int M>
 __global__ void __launch_bounds__(128) k_adaptive(DevEnsemble E, const __grid_constant__ KParams P, Scratch* S) {
-  if (blockIdx.x < gridDim.x / 2) particle_body<M, 0, true>(E, P, S);
-  else gc_body<M, 0, 0, true, false>(E, P, S);
+  const unsigned pb = particle_blocks(P, S), warps = blockDim.x / 32;
+  if (blockIdx.x < pb) particle_body<M, 0, true>(E, P, S, (gridDim.x - pb) * warps);
+  else gc_body<M, 0, 0, true, false>(E, P, S, pb * warps);
 }
 
 }  // namespace rapt

@@ -61,3 +61,36 @@ def test_a_step_budget_bounds_a_launch(cfg):
     st = _sheet(which, max_rows=256, max_steps_per_launch=100, **cfg).advance("adaptive", 20.0)
     assert st["done"] == n and st["failed"] == 0
     assert st["launches"] > 4 and st["kernel_ms"] < 60.0 * st["launches"], (st["kernel_ms"], st["launches"])
+
+
+@pytest.mark.parametrize("n", [90000, 60000])
+def test_one_mode_and_a_few_of_the_other(n):
+    """Nearly all tracers in one mode (above 77,824 on 152 SMs most blocks are given to it)
+    and a few that switch: states, counts and switches of one launch sequence per tracer."""
+    from rapt_gb300 import Ensemble
+    w = W.config4(n, 31)
+    rng = np.random.default_rng(3)
+    d = w["vel"] / np.linalg.norm(w["vel"], axis=1)[:, None]
+    ke = 10 ** rng.uniform(4, 5, n)
+    ke[:: n // 300] = 10 ** rng.uniform(6, 7, len(ke[:: n // 300]))  # protons that change between the modes
+    mass = np.full(n, W.m_el)
+    charge = np.full(n, -W.e)
+    mass[:: n // 300] = W.m_pr
+    charge[:: n // 300] = W.e
+    vel = d * W.speed_from_ke(ke, mass)[:, None]
+    out = []
+    for idx in (np.arange(n), np.arange(n)[:: n // 300]):
+        ens = Ensemble(F.EarthDipole(), len(idx), max_rows=256, max_switch=32)
+        ens.configure(rtol=1e-7, atol=1e-7, gctimestep=0.02, per_tracer_launches=int(len(idx) < n))
+        ens.set_particles(w["pos"][idx], vel[idx], 0.0, mass[idx], charge[idx])
+        ens.upload()
+        ens.adaptive_init()
+        st = ens.advance("adaptive", 0.5)
+        h = ens.download()
+        if len(idx) == n:
+            assert st["accepted"] == h["naccept"].sum() and st["switches"] == h["nswitch"].sum() and st["launches"] == 1
+            assert (h["status"] == 0).sum() > n - 400
+        out.append([h[a].copy() for a in ("s", "t_row", "tcur", "mu", "status", "mode", "naccept", "nreject", "nfcn", "nswitch")])
+    assert out[1][-1].sum() > 10
+    for a, b in zip(*out):
+        assert np.array_equal(a[..., :: n // 300], b, equal_nan=a.dtype.kind == "f")
