@@ -151,9 +151,11 @@ __device__ __noinline__ int fl_trace_dir(const FieldP& f, double t0, const doubl
         S[idx] = s;
         Bs[idx] = mag;
       }
-      if (h != ds || r > quarter * tol) h = dm(h, fmin(fmax(dm(0.84, pow(tol / r, 0.25)), 0.1), 4.0));
-      if (h > ds) h = ds;
-      else if (h < hmin) { raised = true; break; }
+      if (h != ds || r > quarter * tol) {  // else the factor takes h above hmax, which caps it
+        h = dm(h, fmin(fmax(dm(0.84, pow(tol / r, 0.25)), 0.1), 4.0));
+        if (h > ds) h = ds;
+        else if (h < hmin) { raised = true; break; }  // not asked of a capped step (ds may be below hmin)
+      }
     }
     if (raised) return before;
     if (mag > Bm) break;
