@@ -8,6 +8,9 @@ replay of the rounds or one launch sequence per round). ``tune`` times the
 candidate shapes on a sample of the caller's workload -- the arithmetic of every
 tracer is the same under every shape, so device time alone decides -- and
 caches the winner per (field model, run kind, form, tableau) in a JSON file.
+The library's own shape (threads_per_block = blocks_per_sm = 0) is the first
+candidate: a kernel may have shapes that cannot be asked for by number (the FP32
+guiding-centre blocks of up to 1,024 threads whose warps keep in step).
 """
 import json
 import os
@@ -18,6 +21,7 @@ CACHE = os.path.join(os.environ.get("XDG_CACHE_HOME", os.path.join(os.path.expan
                      "rapt_gb300", "autotune.json")
 BLOCKS = (32, 64, 128)
 BLOCKS_PER_SM = (1, 2, 4, 8, 16)
+VERSION = 2  # of the kernels' launch shapes: results cached under another are timed again
 
 
 def cache_key(model, kind, form, tableau):
@@ -40,9 +44,11 @@ def save_cache(table, path=CACHE):
     os.replace(tmp, path)
 
 
-def candidates(blocks=BLOCKS, blocks_per_sm=BLOCKS_PER_SM, graph=(0, 1)):
-    return [dict(threads_per_block=b, blocks_per_sm=m, use_graph=g) for b in blocks for m in blocks_per_sm
-            for g in graph]
+def candidates(blocks=None, blocks_per_sm=None, graph=(0, 1)):
+    """Launch shapes to time: those given, or the library's own shape and all others."""
+    own = [(0, 0)] if blocks is None and blocks_per_sm is None else []
+    shapes = own + [(b, m) for b in blocks or BLOCKS for m in blocks_per_sm or BLOCKS_PER_SM]
+    return [dict(threads_per_block=b, blocks_per_sm=m, use_graph=g) for b, m in shapes for g in graph]
 
 
 def tune(ens, kind, delta, cands=None, key=None, path=CACHE, use_cache=True):
@@ -53,7 +59,7 @@ def tune(ens, kind, delta, cands=None, key=None, path=CACHE, use_cache=True):
     table of device ms per candidate); with a key, the best shape is cached."""
     if key is not None and use_cache:
         hit = load_cache(path).get(key)
-        if hit:
+        if hit and hit.get("version") == VERSION:
             return hit["best"], hit["table"]
     cands = cands or candidates()
     init = {k: v.copy() for k, v in ens.h.items()}
@@ -80,7 +86,7 @@ def tune(ens, kind, delta, cands=None, key=None, path=CACHE, use_cache=True):
     ens.configure(**base)
     if key is not None:
         t = load_cache(path)
-        t[key] = {"best": best, "table": table}
+        t[key] = {"best": best, "table": table, "version": VERSION}
         save_cache(t, path)
     return best, table
 
