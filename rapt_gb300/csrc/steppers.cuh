@@ -222,11 +222,14 @@ __device__ __forceinline__ void dopri5_attempt_rolled(const F& f, double x, cons
   double e = 0.0;
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
-    const double ei = (e1 * k1[i] + e3 * k3[i] + e4 * k4[i] + e5 * k5[i] + e6 * k6[i] + e7 * k7[i]) * h;
+    // sums of products: which product is rounded by itself is spelled out, as the accept
+    // decisions and the rows have to be the same in every kernel that this is inlined into
+    const double ei = fma(e7, k7[i], fma(e6, k6[i], fma(e5, k5[i], fma(e4, k4[i], fma(e1, k1[i], e3 * k3[i]))))) * h;
     const double sk = atol + rtol * fmax(fabs(y[i]), fabs(y1[i]));
     const double r = ei / sk;
     e += r * r;
-    if (DENSE) dd[i] = h * (d1 * k1[i] + d3 * k3[i] + d4 * k4[i] + d5 * k5[i] + d6 * k6[i] + d7 * k7[i]);
+    if (DENSE)
+      dd[i] = h * fma(d7, k7[i], fma(d6, k6[i], fma(d5, k5[i], fma(d4, k4[i], fma(d1, k1[i], d3 * k3[i])))));
   }
   err = sqrt(e * (1.0 / NV));
 }
@@ -241,9 +244,9 @@ __device__ __forceinline__ void dopri5_dense(const double* y0, const double* y1,
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
     const double ydiff = y1[i] - y0[i];
-    const double bspl = h * k1[i] - ydiff;
-    const double r4 = ydiff - h * k7[i] - bspl;
-    out[i] = y0[i] + theta * (ydiff + th1 * (bspl + theta * (r4 + th1 * dd[i])));
+    const double bspl = fma(h, k1[i], -ydiff);
+    const double r4 = fma(-h, k7[i], ydiff) - bspl;
+    out[i] = fma(theta, fma(th1, fma(theta, fma(th1, dd[i], r4), bspl), ydiff), y0[i]);
   }
 }
 
