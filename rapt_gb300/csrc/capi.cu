@@ -41,7 +41,7 @@ struct Ctx {
   cudaStream_t side = nullptr;
   cudaEvent_t fork = nullptr, join = nullptr;
   int8_t* mode0 = nullptr;  // modes at the start of a round (in block)
-  ModelTable tab[RAPT_N_MODELS];
+  ModelTable tab[RAPT_N_MODELS] = {};
   // step-size MLP: one device block of parameters, Adam moments, gradient,
   // loss and packed weights; a separate sample buffer
   void* mlp_block = nullptr;
@@ -837,14 +837,13 @@ static int advance_impl(Ctx* c, int kind, const double* delta, double delta_all,
   // blocks in step: one on every SM, over which the tracers are dealt out
   const int grid_g = block_g > block ? c->num_sms * bps_g : grid_of(bps_g, P.lanes_g, block_g);
 
-  // Guiding centres in the plain form, from one warp a sub-partition up to 32: tracers
-  // shared between the warps at the end of the launch (k_gc_share, k_gc_dense<M, true>).
-  // One block an SM at least, so that every sub-partition has a warp that takes (two:
-  // 10,000 tracers 10.4 -> 12.5 ms, they share the FP64 pipe). Above 32 warps a
-  // sub-partition the end of the launch is 1 % of it. Not in a grid with dense output (the
-  // compiler contracts a row's sums differently in the two kernels, by one unit in the last
-  // place, and a grid's steps follow it); not with a step budget, whose lanes stop between
-  // intervals; without memory for it the plain kernel runs.
+  // Guiding centres in the plain form, from one round of teams a sub-partition up to 32
+  // warps: tracers shared between the warps at the end of the launch (k_gc_share,
+  // k_gc_dense<M, true>). One block an SM at least, so that every sub-partition has a warp
+  // that takes (two: 10,000 tracers 10.4 -> 12.5 ms, they share the FP64 pipe). Above 32
+  // warps a sub-partition the end of the launch is 1 % of it. Not in a grid with dense
+  // output, for which no sharing kernel is built; not with a step budget, whose lanes stop
+  // between intervals; without memory for it the plain kernel runs.
   int grid_s = 0;
   size_t share_head = 0;  // bytes of the mailboxes and the ring
   if (can_share && P.lanes_g == 32) {

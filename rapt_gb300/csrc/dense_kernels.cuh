@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(128) k_gc_dense(DevEnsemble E, const __grid_co
     if (idx >= 0) {
       bool more = seg_ok && t_row < stop;
       if (!more) {
-        if (P.kind == RAPT_KIND_ADAPTIVE && status != RAPT_ST_NONFINITE && status != RAPT_ST_BAD_INPUT &&
+        if (!SHARE && P.kind == RAPT_KIND_ADAPTIVE && status != RAPT_ST_NONFINITE && status != RAPT_ST_BAD_INPUT &&
             status != RAPT_ST_OUT_OF_GRID && status != RAPT_ST_RKF_HMIN && tcur < delta) {
           if (nseg + 1 >= P.max_segments) {
             status = RAPT_ST_ADAPTIVE_LIMIT;
@@ -242,7 +242,7 @@ __global__ void __launch_bounds__(128) k_gc_dense(DevEnsemble E, const __grid_co
             h = 0.0;
             row_end = true;
             if (nonadi) {
-              if (P.kind == RAPT_KIND_ADAPTIVE) {
+              if (!SHARE && P.kind == RAPT_KIND_ADAPTIVE) {  // sharing: guiding centres alone
                 double s6[6];
                 gc_to_particle<M>(P.f, t_row, y, mu, mass, charge, s6);
 #pragma unroll

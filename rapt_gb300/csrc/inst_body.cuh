@@ -204,8 +204,10 @@ void RAPT_CAT(register_model_, RAPT_MODEL)(ModelTable* t) {
   t->occ_adaptive = occ_adaptive;
   t->gc_dense = launch_gc_dense<false>;
   t->occ_gc_dense = occ_gc_dense<false>;
-  t->gc_dense_share = launch_gc_dense<true>;
-  t->occ_gc_dense_share = occ_gc_dense<true>;
+  if constexpr (kM != RAPT_GRID) {  // not dispatched for a grid (advance_impl)
+    t->gc_dense_share = launch_gc_dense<true>;
+    t->occ_gc_dense_share = occ_gc_dense<true>;
+  }
   t->bc_start = bc_start;
   t->bc_interval = bc_interval;
   t->bc_eval = bc_eval;

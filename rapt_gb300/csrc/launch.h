@@ -79,7 +79,7 @@ struct ModelTable {
   OccFn occ_adaptive;
   LaunchFn gc_dense;  // DOPRI5 guiding centres with dense output (rapt_config.dense_output)
   OccFn occ_gc_dense;
-  LaunchFn gc_dense_share;
+  LaunchFn gc_dense_share;  // null for a grid
   OccFn occ_gc_dense_share;
   BcStartFn bc_start;        // BounceCenter.advance: cadence and row count
   BcIntervalFn bc_interval;  // BounceCenter.advance: one output interval of every tracer
