@@ -229,8 +229,10 @@ __device__ __forceinline__ double pow_fp64(double x, double a) {
   return exp2_fp64(a * log2_fp64(x));
 }
 
-// x^(-1/16) for normal x > 0: an FP32 seed (relative error 2^-22 or less) and one
-// step of the binomial series in e = 1 - x y^16 (next term 0.03 e^3, below 1e-17);
+// x^(-1/16) for normal x > 0: an FP32 seed and one step of the binomial series in
+// e = 1 - x y^16. The seed's relative error grows with |log2 x|, whose FP32 sum rounds:
+// 2^-22 up to exponents of 90, 2^-20 up to 300, 2^-19.4 beyond; the next term, 0.023 e^3,
+// is then 2e-18, 4e-17 and 3e-16 (and a starting step needs no more than its first digits).
 // 9 FP64 instructions where exp2(a log2 x) takes some 45.
 __device__ __forceinline__ double rsixteenth_root(double x) {
   const int hi = __double2hiint(x);
