@@ -765,10 +765,12 @@ static int advance_impl(Ctx* c, int kind, const double* delta, double delta_all,
     return fail(c, RAPT_ERR_INVALID, "dense output needs max_rows >= 18 (a step may cover 17 output times)");
   // k_gc32 takes one block an SM, as large as the ensemble fills, whose warps keep in
   // step (fp32_kernels.cuh): from 512 threads on, below which a sub-partition has too few
-  // of the block's warps to gain. Not where a block size is asked for, nor in Adaptive
-  // rounds, where the particle kernel has to find room on the same SMs.
+  // of the block's warps to gain. Not where a block size or a number of blocks an SM is
+  // asked for (it says how much of an SM the launch may take), nor in Adaptive rounds,
+  // where the particle kernel has to find room on the same SMs.
   int block_g = block;
-  if (f32 && kind == RAPT_KIND_GC && c->cfg.threads_per_block <= 0 && !c->cfg.per_tracer_launches) {
+  if (f32 && kind == RAPT_KIND_GC && c->cfg.threads_per_block <= 0 && c->cfg.blocks_per_sm <= 0 &&
+      !c->cfg.per_tracer_launches) {
     const int64_t fill = 128 * ((c->n + 128 * c->num_sms - 1) / (128 * (int64_t)c->num_sms));
     if (fill >= 512) block_g = (int)std::min<int64_t>(1024, fill);
   }
