@@ -47,18 +47,22 @@ FLOPS_PER_ACCEPTED_STEP = 6 * 446 + 275 + 6 * 23 + 4
 # FP32-pipe thread instructions (FFMA + FADD + FMUL) per accepted step of the
 # learned + FP32 guiding-centre kernel k_gc32<DoubleDipole, learned> (the
 # headline form): the float-float stages and centre field, the FP32 stencil
-# differences, the equations and the step learner, from one ncu capture of the
-# 262,144-tracer case (sm__sass_thread_inst_executed_op_{ffma,fadd,fmul}_pred_on.sum
-# over the launch's accepted steps; profiles/k_gc32_learned_doubledipole_262k_full.md).
-FP32_OPS_PER_ACCEPTED_STEP = 9575
+# differences, the equations and the step learner, from an ncu capture of
+# 262,144 tracers in blocks of 128, where only lanes with an attempt to make go
+# through it (sm__sass_thread_inst_executed_op_{ffma,fadd,fmul}_pred_on.sum over
+# the launch's accepted steps). In the blocks whose warps keep in step, the ones
+# timed here, lanes without an attempt go along: 10,971 executed, of which the
+# rest is not counted as work (profiles/k_gc32_learned_doubledipole_262k_full.md).
+FP32_OPS_PER_ACCEPTED_STEP = 9533
 # DRAM traffic of one k_gc32 launch per tracer and simulated second
-# (dram__bytes_read.sum + dram__bytes_write.sum of the same capture: local-memory
+# (dram__bytes_read.sum + dram__bytes_write.sum of the capture in step: local-memory
 # traffic; the algorithmic state traffic is ~464 B per tracer and launch).
-TRAFFIC_PER_TRACER_SECOND = 1.532e5
+TRAFFIC_PER_TRACER_SECOND = 1.460e5
 # Pipe and issue utilisation of the same capture: the headline kernel saturates
-# neither pipe, and instruction fetch is its top stall (the bound it is on).
-HEADLINE_NCU = {"issue_active": 0.482, "fp32_pipe_active": 0.354, "fp64_pipe_active": 0.303,
-                "top_stall": "no_instruction"}
+# neither pipe; of the stalls (warps that were ready apart) local-memory latency
+# comes first, before fixed latencies and the barriers of the stage groups.
+HEADLINE_NCU = {"issue_active": 0.559, "fp32_pipe_active": 0.404, "fp64_pipe_active": 0.296,
+                "top_stall": "long_scoreboard"}
 # FP64 FMA issue rate of a GB300 SM (thread-instructions per clock; ncu's FP64
 # pipe peak, 304 per clock over the 152 SMs).
 FP64_FMA_PER_CLK_PER_SM = 2

@@ -236,11 +236,11 @@ int rapt_gc_bounce_period(void* ctx, int64_t n, const double* state, double* out
 
 /* --- BounceCenter (rapt/BounceCenter.py) and the second invariant ----------
  * BounceCenter.advance(delta) (BounceCenter.py:214-252) for n bounce centres at
- * once, a team of 16 lanes each (six field lines in two directions at a time, in scratch slots
- * of 8 KB a line and direction, in passes of 4,096 tracers; a tracer that meets a non-finite
- * value is rerun with 64 KB slots): the
+ * once, a team of 16 lanes each (six field lines in two directions at a time, in a scratch slot
+ * of 8 KB a line, in passes of 4,096 tracers; a tracer that meets a non-finite value is rerun
+ * with 64 KB slots): the
  * drift gamma m v^2 / (q S_b |B|^2) (grad I x B) with S_b = halfbouncepath
- * and grad I = flutils.gradI (five field-line traces per right-hand side),
+ * and grad I = flutils.gradI (six field lines a right-hand side),
  * rows every bctimestep x the bounce period at the start, SciPy-dopri5
  * restarts per row (config rtol, atol, nsteps; fieldlineresolution).
  *   state[n][5] in/out = (t, x, y, z, tcur): t, x, y, z = trajectory[-1]
